@@ -130,8 +130,36 @@ def _workload(case):
         specular_envmap_size=case.get("specular", 0))
 
 
+def _lit_scene(workload, seed):
+    """The first scene of the seed's series whose lights reach into the room
+    (a spot light that hangs right above a box lights only the box's top,
+    which nothing the camera sees faces): its seed."""
+    k = np.arange(48)
+    phi, tilt = k * 2.399963, np.radians(26.0) * np.sqrt((k + 0.5) / 48)
+    for s in range(seed * 16, seed * 16 + 16):
+        hf = pipeline.host_frame(workload, s)
+        lo = np.array([hf.boxes[b].min[:] for b in range(hf.scene.n_boxes)], np.float64)
+        hi = np.array([hf.boxes[b].max[:] for b in range(hf.scene.n_boxes)], np.float64)
+        reach = []
+        for light in hf.light_descs:
+            o, d = np.array(light.position[:], np.float64), np.array(light.direction[:], np.float64)
+            u = np.cross(d, [1.0, 0.0, 0.0])
+            u /= np.linalg.norm(u)
+            v = np.cross(d, u)
+            rays = np.cos(tilt)[:, None] * d + np.sin(tilt)[:, None] * (np.cos(phi)[:, None] * u + np.sin(phi)[:, None] * v)
+            t0, t1 = (lo[None] - o) / rays[:, None], (hi[None] - o) / rays[:, None]
+            near, far = np.minimum(t0, t1).max(-1), np.maximum(t0, t1).min(-1)
+            hit = np.where((near <= far) & (near > 0), near, np.inf)
+            hit[:, 0] = far[:, 0]  # box 0 is the room, seen from inside
+            reach.append(hit.min(1).mean())
+        if np.mean(reach) >= 0.4:
+            break
+    return s
+
+
 def _pipeline(case, seed):
-    hf = pipeline.host_frame(_workload(case), seed)
+    w = _workload(case)
+    hf = pipeline.host_frame(w, _lit_scene(w, seed))
     t16 = case.get("targets16", False)
     if t16:
         hf.config.output_format = abi.OUTPUT_RGBA16F
@@ -259,7 +287,8 @@ def prepare(case, seed):
         scratch = torch.empty(load().drv_surrogate_train_scratch_floats(case["samples"]), device="cuda")
         return {"kind": kind, "X": X, "Y": Y, "params": params, "m": m, "v": v, "scratch": scratch,
                 "loss": torch.zeros(2, device="cuda"), "step": 500}
-    specs = [(w, seed * 64 + i) for i, (w, _) in enumerate(batch.batch_workloads(case["scenes"], case["first"]))]
+    specs = [(w, _lit_scene(w, seed * 8 + i))
+             for i, (w, _) in enumerate(batch.batch_workloads(case["scenes"], case["first"]))]
     scenes = batch.make_scenes(specs)
     return {"kind": kind, "scenes": scenes, "batch": batch.Batch(scenes, case["streams"], _render_stream())}
 
