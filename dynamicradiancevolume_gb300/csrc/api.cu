@@ -50,7 +50,7 @@ void release(Context* c) {
   cudaFree(c->vox_records);
   cudaFree(c->ndc);
   cudaFree(c->srgb);
-  cudaFree(c->raster_keys);
+  cudaFree(c->raster_mem);
   cudaFree(c->spec_env);
   cudaFree(c->spec_half);
 
@@ -260,7 +260,7 @@ drv_status drv_create(const DrvConfig* cfg, DrvContext** out) {
   // Voxel level 0 (bitmask) and FP32 mips.
   const int N = cfg->voxel_res;
   c->voxel_words = (size_t)N * N * N / 32;
-  if ((e = cudaMalloc(&c->voxel_bits, c->voxel_words * 4)) != cudaSuccess) return bail(e);
+  if ((e = cudaMalloc(&c->voxel_bits, c->voxel_words * 4 + 16 + drv::tile_queue_bytes())) != cudaSuccess) return bail(e);
   c->n_voxel_levels = ilog2(N) + 1;
   size_t off = 0;
   for (int l = 1; l < c->n_voxel_levels; ++l) {
@@ -494,10 +494,13 @@ drv_status ensure_raster_keys(DrvContext* ctx, size_t pixels) {
   if (cs != cudaStreamCaptureStatusNone)
     return fail(ctx, DRV_ERR_INVALID_ARG, "first mesh raster at this size while the stream is being captured");
   DRV_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->s()));
-  cudaFree(ctx->raster_keys);
-  ctx->raster_keys = nullptr;
+  cudaFree(ctx->raster_mem);
+  ctx->raster_mem = nullptr;
   ctx->raster_keys_cap = 0;
-  DRV_TRY_CUDA(ctx, cudaMalloc(&ctx->raster_keys, pixels * sizeof(unsigned long long)));
+  const size_t keys = ((pixels + 2) * sizeof(unsigned long long) + 15) & ~(size_t)15;  // the list's head, the keys
+  DRV_TRY_CUDA(ctx, cudaMalloc(&ctx->raster_mem, keys + drv::tile_queue_bytes()));
+  ctx->raster_keys = static_cast<unsigned long long*>(ctx->raster_mem) + 2;
+  ctx->raster_big = reinterpret_cast<uint4*>(static_cast<char*>(ctx->raster_mem) + keys);
   ctx->raster_keys_cap = pixels;
   return DRV_OK;
 }
@@ -514,7 +517,7 @@ drv_status drv_raster_gbuffer(DrvContext* ctx, const DrvMesh* mesh, const DrvCam
   const drv::RayFrame rf = drv::make_ray_frame(cam->position, cam->direction, cam->up, ty * cam->aspect, ty);
   return cuda_check(ctx,
                     drv::launch_raster_gbuffer(ctx->s(), *mesh, rf, frame->view_projection, w, h, ctx->raster_keys,
-                                               *out, ctx->num_sms),
+                                               ctx->raster_big, *out, ctx->num_sms),
                     "raster_gbuffer");
 }
 
@@ -525,7 +528,8 @@ drv_status drv_raster_rsm(DrvContext* ctx, const DrvMesh* mesh, const DrvSpotLig
   const size_t R = (size_t)light->rsm_render_resolution;
   drv_status st = ensure_raster_keys(ctx, R * R);
   if (st != DRV_OK) return st;
-  return cuda_check(ctx, drv::launch_raster_rsm(ctx->s(), *mesh, *light, ctx->raster_keys, *out, ctx->num_sms),
+  return cuda_check(ctx, drv::launch_raster_rsm(ctx->s(), *mesh, *light, ctx->raster_keys, ctx->raster_big, *out,
+                                                ctx->num_sms),
                     "raster_rsm");
 }
 

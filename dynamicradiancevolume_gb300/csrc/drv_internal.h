@@ -178,11 +178,15 @@ struct Context {
   uint32_t* mips_ticket() const { return scratch_words + 5; }
   uint32_t* input_err() const { return scratch_words + 4; }
   // Voxels.
-  uint32_t* voxel_bits = nullptr;
+  uint32_t* voxel_bits = nullptr;  // followed by the tile list of drv_voxelize_triangles: head (16 bytes), entries
   size_t voxel_words = 0;
   float* ndc = nullptr;  // NDC x of each pixel column (width), then y of each row (height): allocation
   float* srgb = nullptr;  // the GL sRGB decode of the 256 byte values (DRV_ALBEDO_SRGB8)
-  unsigned long long* raster_keys = nullptr;  // mesh producers' per-pixel visibility (drv_raster_*)
+  // Mesh producers (drv_raster_*): one allocation of the large triangles'
+  // tile list head (16 bytes), the per-pixel visibility keys, the list.
+  void* raster_mem = nullptr;
+  unsigned long long* raster_keys = nullptr;
+  uint4* raster_big = nullptr;
   size_t raster_keys_cap = 0;
   uint8_t* vox_corners = nullptr;  // level 0, corner-packed bytes, x fastest
   void* mips = nullptr;  // levels 1..L concatenated: float (FP32 precision) or half (BF16 precision)
@@ -252,9 +256,9 @@ cudaError_t launch_raycast_gbuffer(cudaStream_t s, const DrvBox* boxes, int n_bo
                                    const float* view_proj, int w, int h, DrvGBufferOut out);
 cudaError_t launch_raycast_rsm(cudaStream_t s, const DrvBox* boxes, int n_boxes, const DrvSpotLight& L, DrvRSMOut out);
 cudaError_t launch_raster_gbuffer(cudaStream_t s, const DrvMesh& mesh, RayFrame rf, const float* view_proj, int w,
-                                  int h, unsigned long long* keys, DrvGBufferOut out, int num_sms);
+                                  int h, unsigned long long* keys, uint4* big, DrvGBufferOut out, int num_sms);
 cudaError_t launch_raster_rsm(cudaStream_t s, const DrvMesh& mesh, const DrvSpotLight& L, unsigned long long* keys,
-                              DrvRSMOut out, int num_sms);
+                              uint4* big, DrvRSMOut out, int num_sms);
 // Up to three RSM downsample passes res -> res/2 -> ... in one launch;
 // fo/no/dlo[k] receive level k + 1 (F32 flux and (d, d^2), RG16I normals).
 cudaError_t launch_rsm_chain(cudaStream_t s, int res, int passes, const void* flux, const int16_t* nrm,
@@ -266,6 +270,9 @@ cudaError_t launch_voxelize(cudaStream_t s, const DrvBox* boxes, int n_boxes, co
                             uint32_t* bits);
 cudaError_t launch_voxelize_triangles(cudaStream_t s, const float* positions, int n_vertices, const uint32_t* indices,
                                       int n_triangles, const DrvVolumeInfo& vol, int n, uint32_t* bits, int num_sms);
+// Bytes of the large triangles' list (tile_queue.cuh): behind the voxel bits
+// (with a 16-byte head) and behind the raster keys (the head before them).
+size_t tile_queue_bytes();
 // ticket: a zeroed word of the context's (the last CTA builds the levels
 // above one 32^3 block and zeroes it again).
 cudaError_t launch_build_mips(cudaStream_t s, int n, const uint32_t* bits, void* mips, const size_t* offsets,

@@ -2,10 +2,10 @@
 // (fillgbuffer.frag) and the RSM fill (fillrsm.frag:24-62) of an arbitrary
 // mesh, untextured (linear RGB albedo per triangle, optional vertex normals).
 //
-// Two passes per target. Visibility: a warp per triangle projects it with the
-// target's view-projection (row-major M v), clips it against the near plane
+// Two passes per target. Visibility: each triangle is projected with the
+// target's view-projection (row-major M v) and clipped against the near plane
 // (reversed-Z: z/w <= 1, i.e. w - z >= 0; a polygon of up to 4 vertices,
-// drawn as a fan), and for every pixel centre inside with depth in [0, 1]
+// drawn as a fan), and every pixel centre inside with depth in [0, 1]
 // takes the 64-bit maximum of (depth bits, triangle + 1) — reversed-Z, the
 // nearest surface has the largest depth; equal depths go to the higher
 // triangle index. Coverage is watertight: each edge function is evaluated with
@@ -19,6 +19,7 @@
 // fillrsm.frag at the hit point.
 #include "drv_device.cuh"
 #include "drv_internal.h"
+#include "tile_queue.cuh"
 
 namespace drv {
 namespace {
@@ -75,62 +76,176 @@ __device__ __forceinline__ float edge_fn(float ax, float ay, float bx, float by,
   return swap ? -e : e;
 }
 
-// Visibility pass: a warp per triangle (grid-stride).
-__global__ void __launch_bounds__(256) raster_kernel(MeshView m, Mat4 M, int W, int H,
-                                                     unsigned long long* __restrict__ keys) {
-  const int lane = threadIdx.x & 31;
-  const int n_warps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < m.nt; k += n_warps) {
-    uint32_t vi[3];
-    if (!tri_indices(m, k, vi)) continue;
-    const float4 c[3] = {to_clip(M, vertex(m, vi[0])), to_clip(M, vertex(m, vi[1])), to_clip(M, vertex(m, vi[2]))};
-    // Clip against the near plane (Sutherland-Hodgman, one plane). The cut
-    // point is interpolated from the inside end, so the two triangles sharing
-    // a cut edge compute the same vertex.
-    float4 poly[4];
+// A screen triangle: its vertices (pixels, reversed-Z depth) and clamped
+// pixel bounding box.
+struct ScreenTri {
+  float x[3], y[3], z[3];
+  int bx0, by0, bx1, by1;
+};
+
+// Fan triangle f (1 or 2) of triangle k clipped against the near plane
+// (Sutherland-Hodgman, one plane; the cut point is interpolated from the
+// inside end, so the two triangles sharing a cut edge compute the same
+// vertex). False when there is none, it has no area, or it misses the target.
+__device__ __forceinline__ bool screen_triangle(const MeshView& m, const Mat4& M, int k, int f, int W, int H,
+                                                ScreenTri& t) {
+  uint32_t vi[3];
+  if (!tri_indices(m, k, vi)) return false;
+  const float4 c[3] = {to_clip(M, vertex(m, vi[0])), to_clip(M, vertex(m, vi[1])), to_clip(M, vertex(m, vi[2]))};
+  float4 poly[3] = {c[0], c[1], c[2]};  // the fan's vertices 0, f, f + 1
+  const float d[3] = {near_distance(c[0]), near_distance(c[1]), near_distance(c[2])};
+  if (d[0] >= 0.0f && d[1] >= 0.0f && d[2] >= 0.0f) {
+    if (f != 1) return false;
+  } else {
     int n = 0;
+    bool have[3] = {false, false, false};
+    auto put = [&](float4 p) {
+      if (n == 0) poly[0] = p, have[0] = true;
+      if (n == f) poly[1] = p, have[1] = true;
+      if (n == f + 1) poly[2] = p, have[2] = true;
+      ++n;
+    };
+#pragma unroll
     for (int e = 0; e < 3; ++e) {
       const float4 a = c[e], b = c[(e + 1) % 3];
-      const float da = near_distance(a), db = near_distance(b);
+      const float da = d[e], db = d[(e + 1) % 3];
       const bool ia = da >= 0.0f, ib = db >= 0.0f;
-      if (ia) poly[n++] = a;
-      if (ia != ib) poly[n++] = ia ? lerp4(a, b, da / (da - db)) : lerp4(b, a, db / (db - da));
+      if (ia) put(a);
+      if (ia != ib) put(ia ? lerp4(a, b, da / (da - db)) : lerp4(b, a, db / (db - da)));
     }
-    if (n < 3) continue;
-    float sx[4], sy[4], sz[4];
-    for (int i = 0; i < n; ++i) {
-      const float iw = __fdiv_rn(1.0f, poly[i].w);
-      sx[i] = __fmul_rn(__fmaf_rn(__fmul_rn(poly[i].x, iw), 0.5f, 0.5f), (float)W);
-      sy[i] = __fmul_rn(__fmaf_rn(__fmul_rn(poly[i].y, iw), 0.5f, 0.5f), (float)H);
-      sz[i] = __fmul_rn(poly[i].z, iw);
+    if (!(have[0] && have[1] && have[2])) return false;
+  }
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float iw = __fdiv_rn(1.0f, poly[i].w);
+    t.x[i] = __fmul_rn(__fmaf_rn(__fmul_rn(poly[i].x, iw), 0.5f, 0.5f), (float)W);
+    t.y[i] = __fmul_rn(__fmaf_rn(__fmul_rn(poly[i].y, iw), 0.5f, 0.5f), (float)H);
+    t.z[i] = __fmul_rn(poly[i].z, iw);
+  }
+  const float area = edge_fn(t.x[0], t.y[0], t.x[1], t.y[1], t.x[2], t.y[2]);
+  if (!(area != 0.0f)) return false;
+  t.bx0 = max(0, (int)floorf(fminf(fminf(t.x[0], t.x[1]), t.x[2])));
+  t.by0 = max(0, (int)floorf(fminf(fminf(t.y[0], t.y[1]), t.y[2])));
+  t.bx1 = min(W - 1, (int)floorf(fmaxf(fmaxf(t.x[0], t.x[1]), t.x[2])));
+  t.by1 = min(H - 1, (int)floorf(fmaxf(fmaxf(t.y[0], t.y[1]), t.y[2])));
+  return t.bx1 >= t.bx0 && t.by1 >= t.by0;
+}
+
+// The three edge functions of a screen triangle, opposite vertices 0, 1, 2
+// and positive inside, split so that a walk over pixels keeps the parts of a
+// row and of a column: edge_fn's value is u(row) - v(column), with sign +-1.
+struct TriEdges {
+  float x0[3], y0[3], dx[3], dy[3], sign[3], z[3];
+  __device__ __forceinline__ explicit TriEdges(const ScreenTri& t) {
+    const float orient = edge_fn(t.x[0], t.y[0], t.x[1], t.y[1], t.x[2], t.y[2]) > 0.0f ? 1.0f : -1.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int a = (i + 1) % 3, b = (i + 2) % 3;
+      const bool swap = t.x[a] > t.x[b] || (t.x[a] == t.x[b] && t.y[a] > t.y[b]);
+      x0[i] = swap ? t.x[b] : t.x[a];
+      y0[i] = swap ? t.y[b] : t.y[a];
+      dx[i] = __fsub_rn(swap ? t.x[a] : t.x[b], x0[i]);
+      dy[i] = __fsub_rn(swap ? t.y[a] : t.y[b], y0[i]);
+      sign[i] = swap ? -orient : orient;
+      z[i] = t.z[i];
     }
-    for (int f = 1; f + 1 < n; ++f) {  // fan (0, f, f + 1)
-      const float x0 = sx[0], y0 = sy[0], x1 = sx[f], y1 = sy[f], x2 = sx[f + 1], y2 = sy[f + 1];
-      const float area = edge_fn(x0, y0, x1, y1, x2, y2);
-      if (!(area != 0.0f)) continue;
-      const float orient = area > 0.0f ? 1.0f : -1.0f;
-      const int bx0 = max(0, (int)floorf(fminf(fminf(x0, x1), x2))), by0 = max(0, (int)floorf(fminf(fminf(y0, y1), y2)));
-      const int bx1 = min(W - 1, (int)floorf(fmaxf(fmaxf(x0, x1), x2))), by1 = min(H - 1, (int)floorf(fmaxf(fmaxf(y0, y1), y2)));
-      if (bx1 < bx0 || by1 < by0) continue;
-      const int bw = bx1 - bx0 + 1;
-      const int total = bw * (by1 - by0 + 1);
-      for (int q = lane; q < total; q += 32) {
-        const int px = bx0 + q % bw, py = by0 + q / bw;
-        const float cx = (float)px + 0.5f, cy = (float)py + 0.5f;
-        // edge functions opposite vertices 0, f, f+1, made positive inside
-        const float e0 = orient * edge_fn(x1, y1, x2, y2, cx, cy);
-        const float e1 = orient * edge_fn(x2, y2, x0, y0, cx, cy);
-        const float e2 = orient * edge_fn(x0, y0, x1, y1, cx, cy);
-        if (e0 < 0.0f || e1 < 0.0f || e2 < 0.0f) continue;
-        const float sum = e0 + e1 + e2;
-        if (!(sum > 0.0f)) continue;
-        const float z = (e0 * sz[0] + e1 * sz[f] + e2 * sz[f + 1]) / sum;
-        if (!(z >= 0.0f && z <= 1.0f)) continue;
-        const unsigned long long key = (unsigned long long)__float_as_uint(z) << 32 | (unsigned long long)(k + 1);
-        atomicMax(keys + (size_t)py * W + px, key);
+  }
+  __device__ __forceinline__ float row(int i, float cy) const { return __fmul_rn(dx[i], __fsub_rn(cy, y0[i])); }
+  __device__ __forceinline__ float column(int i, float cx) const { return __fmul_rn(dy[i], __fsub_rn(cx, x0[i])); }
+  // The pixel's visibility key of triangle k into its slot, if it is inside.
+  __device__ __forceinline__ void cover(const float (&u)[3], const float (&v)[3], int k,
+                                        unsigned long long* slot) const {
+    const float e0 = sign[0] * __fsub_rn(u[0], v[0]), e1 = sign[1] * __fsub_rn(u[1], v[1]),
+                e2 = sign[2] * __fsub_rn(u[2], v[2]);
+    if (e0 < 0.0f || e1 < 0.0f || e2 < 0.0f) return;
+    const float sum = e0 + e1 + e2;
+    if (!(sum > 0.0f)) return;
+    const float d = (e0 * z[0] + e1 * z[1] + e2 * z[2]) / sum;
+    if (!(d >= 0.0f && d <= 1.0f)) return;
+    atomicMax(slot, (unsigned long long)__float_as_uint(d) << 32 | (unsigned long long)(k + 1));
+  }
+  // False when some edge is negative over the whole box: each edge's computed
+  // value is monotone along a row and along a column (every rounding is), so
+  // its largest value over the box is at one of the four corners.
+  __device__ __forceinline__ bool touches(float cx0, float cy0, float cx1, float cy1) const {
+    bool out = false;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float u0 = row(i, cy0), u1 = row(i, cy1), v0 = column(i, cx0), v1 = column(i, cx1);
+      out = out || (sign[i] * __fsub_rn(u0, v0) < 0.0f && sign[i] * __fsub_rn(u0, v1) < 0.0f &&
+                    sign[i] * __fsub_rn(u1, v0) < 0.0f && sign[i] * __fsub_rn(u1, v1) < 0.0f);
+    }
+    return !out;
+  }
+};
+
+__device__ __forceinline__ float bcast(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// Visibility pass. A lane sets up a triangle (grid-stride, kWarpTris
+// consecutive triangles per warp: a setup per lane instead of one per warp);
+// the warp then walks the small ones one after the other, and the large ones
+// go to the tile list for raster_tiles_kernel (figures: tile_queue.cuh). Bound
+// by issue: about 35 instructions per pixel of a bounding box.
+__global__ void __launch_bounds__(256) raster_kernel(MeshView m, Mat4 M, int W, int H,
+                                                     unsigned long long* __restrict__ keys, TileQueue queue) {
+  const int lane = threadIdx.x & 31;
+  const int n_warps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpTris; k0 < m.nt; k0 += n_warps * kWarpTris) {
+#pragma unroll 1
+    for (int f = 1; f <= 2; ++f) {  // fan triangle 2: only of a triangle the near plane cuts
+      ScreenTri t{};
+      bool walk = lane < kWarpTris && k0 + lane < m.nt && screen_triangle(m, M, k0 + lane, f, W, H, t);
+      if (walk && (long long)(t.bx1 - t.bx0 + 1) * (t.by1 - t.by0 + 1) > kDirectPixels)
+        walk = !tile_queue_push(queue, 2u * (uint32_t)(k0 + lane) + (uint32_t)(f - 1),
+                                tile_count(t.bx0, t.by0, t.bx1, t.by1));
+      for (uint32_t todo = __ballot_sync(0xffffffffu, walk); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        ScreenTri b;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) b.x[i] = bcast(t.x[i], src), b.y[i] = bcast(t.y[i], src), b.z[i] = bcast(t.z[i], src);
+        b.bx0 = bcast(t.bx0, src), b.by0 = bcast(t.by0, src), b.bx1 = bcast(t.bx1, src), b.by1 = bcast(t.by1, src);
+        const TriEdges e(b);
+        const int lw = lanes_per_row(b.bx1 - b.bx0 + 1), lx = lane & (lw - 1), ly = lane / lw;
+        for (int py = b.by0 + ly; py <= b.by1; py += 32 / lw) {
+          const float cy = (float)py + 0.5f;
+          const float u[3] = {e.row(0, cy), e.row(1, cy), e.row(2, cy)};
+          for (int px = b.bx0 + lx; px <= b.bx1; px += lw) {
+            const float cx = (float)px + 0.5f;
+            const float v[3] = {e.column(0, cx), e.column(1, cx), e.column(2, cx)};
+            e.cover(u, v, k0 + src, keys + (size_t)py * W + px);
+          }
+        }
       }
     }
   }
+}
+
+// The listed triangles, tile by tile.
+__global__ void __launch_bounds__(256) raster_tiles_kernel(MeshView m, Mat4 M, int W, int H,
+                                                           unsigned long long* __restrict__ keys, TileQueue queue) {
+  const int lane = threadIdx.x & 31;
+  tile_queue_share(queue, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                   [&](uint32_t code, uint32_t tile, uint32_t n) {
+    const int k = (int)(code >> 1);
+    ScreenTri t;
+    if (!screen_triangle(m, M, k, 1 + (int)(code & 1u), W, H, t)) return;
+    const TriEdges e(t);
+    const int columns = tile_columns(t.bx0, t.bx1);
+    for (uint32_t q = tile; q < tile + n; ++q) {
+      const int x0 = (t.bx0 / kTileW + (int)(q % (uint32_t)columns)) * kTileW, px = x0 + lane;
+      const int y0 = t.by0 + (int)(q / (uint32_t)columns) * kTileH, y1 = min(y0 + kTileH - 1, t.by1);
+      if (!e.touches((float)x0 + 0.5f, (float)y0 + 0.5f, (float)(x0 + kTileW - 1) + 0.5f, (float)y1 + 0.5f)) continue;
+      const float cx = (float)px + 0.5f;
+      const float v[3] = {e.column(0, cx), e.column(1, cx), e.column(2, cx)};
+      if (px < t.bx0 || px > t.bx1) continue;
+      for (int py = y0; py <= y1; ++py) {
+        const float cy = (float)py + 0.5f;
+        const float u[3] = {e.row(0, cy), e.row(1, cy), e.row(2, cy)};
+        e.cover(u, v, k, keys + (size_t)py * W + px);
+      }
+    }
+  });
 }
 
 // Hit point of ray (o, d) on the plane of triangle tri, the normal turned
@@ -265,23 +380,28 @@ MeshView mesh_view(const DrvMesh& mesh) {
   return MeshView{mesh.positions, mesh.normals, mesh.albedo, mesh.indices, mesh.n_vertices, mesh.n_triangles};
 }
 
+// keys: the pixels' keys, preceded by the tile list's head (16 bytes, cleared
+// with them).
 cudaError_t raster(cudaStream_t s, const MeshView& m, const float* view_proj, int W, int H, unsigned long long* keys,
-                   int num_sms) {
-  cudaError_t e = cudaMemsetAsync(keys, 0, (size_t)W * H * sizeof(unsigned long long), s);
+                   uint4* big, int num_sms) {
+  const TileQueue queue{keys - 2, big};
+  cudaError_t e = cudaMemsetAsync(queue.head, 0, ((size_t)W * H + 2) * sizeof(unsigned long long), s);
   if (e != cudaSuccess || m.nt <= 0) return e;
   Mat4 M;
   for (int i = 0; i < 16; ++i) M.m[i] = view_proj[i];
-  const int warps = m.nt < num_sms * 64 ? m.nt : num_sms * 64;
-  raster_kernel<<<(warps + 7) / 8, 256, 0, s>>>(m, M, W, H, keys);
+  const int warps = (m.nt - 1) / kWarpTris + 1 < num_sms * 64 ? (m.nt - 1) / kWarpTris + 1 : num_sms * 64;
+  raster_kernel<<<(warps + 7) / 8, 256, 0, s>>>(m, M, W, H, keys, queue);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  raster_tiles_kernel<<<num_sms * 6, 256, 0, s>>>(m, M, W, H, keys, queue);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_raster_gbuffer(cudaStream_t s, const DrvMesh& mesh, RayFrame rf, const float* view_proj, int w,
-                                  int h, unsigned long long* keys, DrvGBufferOut out, int num_sms) {
+                                  int h, unsigned long long* keys, uint4* big, DrvGBufferOut out, int num_sms) {
   const MeshView m = mesh_view(mesh);
-  cudaError_t e = raster(s, m, view_proj, w, h, keys, num_sms);
+  cudaError_t e = raster(s, m, view_proj, w, h, keys, big, num_sms);
   if (e != cudaSuccess) return e;
   Mat4 M;
   for (int i = 0; i < 16; ++i) M.m[i] = view_proj[i];
@@ -291,10 +411,10 @@ cudaError_t launch_raster_gbuffer(cudaStream_t s, const DrvMesh& mesh, RayFrame 
 }
 
 cudaError_t launch_raster_rsm(cudaStream_t s, const DrvMesh& mesh, const DrvSpotLight& L, unsigned long long* keys,
-                              DrvRSMOut out, int num_sms) {
+                              uint4* big, DrvRSMOut out, int num_sms) {
   const MeshView m = mesh_view(mesh);
   const int R = L.rsm_render_resolution;
-  cudaError_t e = raster(s, m, L.view_projection, R, R, keys, num_sms);
+  cudaError_t e = raster(s, m, L.view_projection, R, R, keys, big, num_sms);
   if (e != cudaSuccess) return e;
   dim3 block(16, 16), grid((R + 15) / 16, (R + 15) / 16);
   rsm_resolve_kernel<<<grid, block, 0, s>>>(m, L, keys, out);

@@ -8,6 +8,7 @@
 // 8^l <= 2^24 for N <= 256), so FP32 holds them exactly.
 #include "drv_device.cuh"
 #include "drv_internal.h"
+#include "tile_queue.cuh"
 
 namespace drv {
 namespace {
@@ -199,47 +200,108 @@ struct TriVolume {
   float vs;
 };
 
-// A warp per triangle (grid-stride): every lane forms the same setup, the
-// lanes share the pixels of the grown AABB.
+// What the walk over a triangle's pixels needs of its setup.
+struct TriWalk {
+  float plane[3][3], aabb[4], zA, zB, zC, max_change;
+  int side, x0, y0, x1, y1;
+};
+
+// Triangle k's walk; false when it sets no voxel.
+__device__ __forceinline__ bool tri_walk(const float* __restrict__ pos, int n_vertices,
+                                         const uint32_t* __restrict__ idx, int k, const TriVolume& tv, int N,
+                                         TriWalk& w) {
+  const uint32_t i0 = idx ? __ldg(idx + 3 * k) : 3u * k, i1 = idx ? __ldg(idx + 3 * k + 1) : 3u * k + 1,
+                 i2 = idx ? __ldg(idx + 3 * k + 2) : 3u * k + 2;
+  if (i0 >= (uint32_t)n_vertices || i1 >= (uint32_t)n_vertices || i2 >= (uint32_t)n_vertices) return false;
+  float P[3][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    P[0][a] = __ldg(pos + 3 * (size_t)i0 + a);
+    P[1][a] = __ldg(pos + 3 * (size_t)i1 + a);
+    P[2][a] = __ldg(pos + 3 * (size_t)i2 + a);
+  }
+  const TriSetup t = tri_setup(P[0], P[1], P[2], tv.vm, tv.vs);
+  if (!t.ok) return false;
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) w.plane[e][a] = t.plane[e][a];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) w.aabb[a] = t.aabb[a];
+  w.zA = t.zA, w.zB = t.zB, w.zC = t.zC, w.max_change = t.max_change, w.side = t.side;
+  w.x0 = max(0, (int)floorf(t.aabb[0])), w.y0 = max(0, (int)floorf(t.aabb[1]));
+  w.x1 = min(N - 1, (int)floorf(t.aabb[2])), w.y1 = min(N - 1, (int)floorf(t.aabb[3]));
+  return w.x1 >= w.x0 && w.y1 >= w.y0;
+}
+
+__device__ __forceinline__ void tri_pixel(const TriWalk& t, int px, int py, int N, uint32_t* __restrict__ bits) {
+  const float cx = dadd((float)px, 0.5f), cy = dadd((float)py, 0.5f);
+  if (cx < t.aabb[0] || cy < t.aabb[1] || cx > t.aabb[2] || cy > t.aabb[3]) return;
+  bool in = true;
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+    in = in && dadd(dadd(dmul(t.plane[e][0], cx), dmul(t.plane[e][1], cy)), t.plane[e][2]) <= 0.0f;
+  if (!in) return;
+  const float z = dadd(dadd(dmul(t.zA, cx), dmul(t.zB, cy)), t.zC);
+  if (!(z >= 0.0f && z <= (float)N)) return;
+  const int zi = (int)z;
+  set_voxel_swizzled(bits, N, t.side, px, py, zi);
+  if ((int)dsub(z, t.max_change) != zi) set_voxel_swizzled(bits, N, t.side, px, py, zi - 1);
+  if ((int)dadd(z, t.max_change) != zi) set_voxel_swizzled(bits, N, t.side, px, py, zi + 1);
+}
+
+__device__ __forceinline__ float bcast(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// A lane sets up a triangle (grid-stride, kWarpTris per warp); the warp walks
+// the small ones one after the other, the large ones go to the tile list for
+// triangle_tiles_kernel (figures: tile_queue.cuh).
 __global__ void __launch_bounds__(256) triangles_kernel(const float* __restrict__ pos, int n_vertices,
                                                         const uint32_t* __restrict__ idx, int n_tris, TriVolume tv,
-                                                        int N, uint32_t* __restrict__ bits) {
+                                                        int N, uint32_t* __restrict__ bits, TileQueue queue) {
   const int lane = threadIdx.x & 31;
   const int n_warps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int k = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < n_tris; k += n_warps) {
-    const uint32_t i0 = idx ? __ldg(idx + 3 * k) : 3u * k, i1 = idx ? __ldg(idx + 3 * k + 1) : 3u * k + 1,
-                   i2 = idx ? __ldg(idx + 3 * k + 2) : 3u * k + 2;
-    if (i0 >= (uint32_t)n_vertices || i1 >= (uint32_t)n_vertices || i2 >= (uint32_t)n_vertices) continue;
-    float P[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      P[0][a] = __ldg(pos + 3 * (size_t)i0 + a);
-      P[1][a] = __ldg(pos + 3 * (size_t)i1 + a);
-      P[2][a] = __ldg(pos + 3 * (size_t)i2 + a);
-    }
-    const TriSetup t = tri_setup(P[0], P[1], P[2], tv.vm, tv.vs);
-    if (!t.ok) continue;
-    const int x0 = max(0, (int)floorf(t.aabb[0])), y0 = max(0, (int)floorf(t.aabb[1]));
-    const int x1 = min(N - 1, (int)floorf(t.aabb[2])), y1 = min(N - 1, (int)floorf(t.aabb[3]));
-    if (x1 < x0 || y1 < y0) continue;
-    const int W = x1 - x0 + 1, total = W * (y1 - y0 + 1);
-    for (int q = lane; q < total; q += 32) {
-      const int px = x0 + q % W, py = y0 + q / W;
-      const float cx = dadd((float)px, 0.5f), cy = dadd((float)py, 0.5f);
-      if (cx < t.aabb[0] || cy < t.aabb[1] || cx > t.aabb[2] || cy > t.aabb[3]) continue;
-      bool in = true;
+  for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpTris; k0 < n_tris; k0 += n_warps * kWarpTris) {
+    TriWalk t{};
+    bool walk = lane < kWarpTris && k0 + lane < n_tris && tri_walk(pos, n_vertices, idx, k0 + lane, tv, N, t);
+    if (walk && (t.x1 - t.x0 + 1) * (t.y1 - t.y0 + 1) > kDirectPixels)
+      walk = !tile_queue_push(queue, (uint32_t)(k0 + lane), tile_count(t.x0, t.y0, t.x1, t.y1));
+    for (uint32_t todo = __ballot_sync(0xffffffffu, walk); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      TriWalk b;
 #pragma unroll
       for (int e = 0; e < 3; ++e)
-        in = in && dadd(dadd(dmul(t.plane[e][0], cx), dmul(t.plane[e][1], cy)), t.plane[e][2]) <= 0.0f;
-      if (!in) continue;
-      const float z = dadd(dadd(dmul(t.zA, cx), dmul(t.zB, cy)), t.zC);
-      if (!(z >= 0.0f && z <= (float)N)) continue;
-      const int zi = (int)z;
-      set_voxel_swizzled(bits, N, t.side, px, py, zi);
-      if ((int)dsub(z, t.max_change) != zi) set_voxel_swizzled(bits, N, t.side, px, py, zi - 1);
-      if ((int)dadd(z, t.max_change) != zi) set_voxel_swizzled(bits, N, t.side, px, py, zi + 1);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) b.plane[e][a] = bcast(t.plane[e][a], src);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) b.aabb[a] = bcast(t.aabb[a], src);
+      b.zA = bcast(t.zA, src), b.zB = bcast(t.zB, src), b.zC = bcast(t.zC, src);
+      b.max_change = bcast(t.max_change, src), b.side = bcast(t.side, src);
+      b.x0 = bcast(t.x0, src), b.y0 = bcast(t.y0, src), b.x1 = bcast(t.x1, src), b.y1 = bcast(t.y1, src);
+      const int lw = lanes_per_row(b.x1 - b.x0 + 1), lx = lane & (lw - 1), ly = lane / lw;
+      for (int py = b.y0 + ly; py <= b.y1; py += 32 / lw)
+        for (int px = b.x0 + lx; px <= b.x1; px += lw) tri_pixel(b, px, py, N, bits);
     }
   }
+}
+
+// The listed triangles, tile by tile.
+__global__ void __launch_bounds__(256) triangle_tiles_kernel(const float* __restrict__ pos, int n_vertices,
+                                                             const uint32_t* __restrict__ idx, TriVolume tv, int N,
+                                                             uint32_t* __restrict__ bits, TileQueue queue) {
+  const int lane = threadIdx.x & 31;
+  tile_queue_share(queue, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                   [&](uint32_t code, uint32_t tile, uint32_t n) {
+    TriWalk t;
+    if (!tri_walk(pos, n_vertices, idx, (int)code, tv, N, t)) return;
+    const int columns = tile_columns(t.x0, t.x1);
+    for (uint32_t q = tile; q < tile + n; ++q) {
+      const int px = (t.x0 / kTileW + (int)(q % (uint32_t)columns)) * kTileW + lane;
+      const int y0 = t.y0 + (int)(q / (uint32_t)columns) * kTileH, y1 = min(y0 + kTileH - 1, t.y1);
+      if (px < t.x0 || px > t.x1) continue;
+      for (int py = y0; py <= y1; ++py) tri_pixel(t, px, py, N, bits);
+    }
+  });
 }
 
 struct MipOffsets {
@@ -533,13 +595,21 @@ cudaError_t launch_voxelize(cudaStream_t s, const DrvBox* boxes, int n_boxes, co
 cudaError_t launch_voxelize_triangles(cudaStream_t s, const float* positions, int n_vertices, const uint32_t* indices,
                                       int n_triangles, const DrvVolumeInfo& vol, int n, uint32_t* bits, int num_sms) {
   if (n < 32 || (n & 31)) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(bits, 0, (size_t)n * n * (n / 32) * sizeof(uint32_t), s);
+  // The large triangles' list lies behind the bits: its head is cleared with them.
+  const size_t words = (size_t)n * n * (n / 32);
+  const TileQueue queue{reinterpret_cast<unsigned long long*>(bits + words), reinterpret_cast<uint4*>(bits + words + 4)};
+  cudaError_t e = cudaMemsetAsync(bits, 0, (words + 4) * sizeof(uint32_t), s);
   if (e != cudaSuccess || n_triangles <= 0) return e;
   TriVolume tv{{vol.volume_world_min[0], vol.volume_world_min[1], vol.volume_world_min[2]}, vol.voxel_size_in_world};
-  const int warps = (n_triangles + 0) < num_sms * 64 ? n_triangles : num_sms * 64;  // <= 64 warps per SM in flight
-  triangles_kernel<<<(warps + 7) / 8, 256, 0, s>>>(positions, n_vertices, indices, n_triangles, tv, n, bits);
+  const int groups = (n_triangles - 1) / kWarpTris + 1;
+  const int warps = groups < num_sms * 64 ? groups : num_sms * 64;  // <= 64 warps per SM in flight
+  triangles_kernel<<<(warps + 7) / 8, 256, 0, s>>>(positions, n_vertices, indices, n_triangles, tv, n, bits, queue);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  triangle_tiles_kernel<<<num_sms * 6, 256, 0, s>>>(positions, n_vertices, indices, tv, n, bits, queue);
   return cudaGetLastError();
 }
+
+size_t tile_queue_bytes() { return (size_t)kTileQueueCap * sizeof(uint4); }
 
 cudaError_t launch_build_mips(cudaStream_t s, int n, const uint32_t* bits, void* mips, const size_t* offsets,
                               int n_levels, int precision, uint32_t* ticket) {
