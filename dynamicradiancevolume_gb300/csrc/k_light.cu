@@ -512,8 +512,17 @@ __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
 // measuring instance): the voxel loads of all cones are summed into
 // counters[1] (level-0 corner bytes), [2] (16-byte mip records) and [7]
 // (plain mip texels).
+// Bound by issue (73% of slots) and the L1's data path (69%: scattered byte and
+// record loads): 1920x1080, 3.9 M cones, 346 -> 286 us with the two-phase march
+// on texture coordinates and the corner table (voxel_sample.cuh; 322 -> 264 M
+// warp instructions). Six CTAs per SM (40 registers) against five: 633 / 642 us
+// for the frame; 128-thread CTAs leave the tables less L1 (651 against 642).
+constexpr int kConeThreads = 256;
 template <bool BF16, bool COUNT = false>
-__global__ void __launch_bounds__(128) cone_kernel(StageParams p, PairList L) {
+__global__ void __launch_bounds__(kConeThreads, 6) cone_kernel(StageParams p, PairList L) {
+  __shared__ SharedTableStorage s_table;
+  const SharedTable table = fill_table(s_table, p.vox);
+  __syncthreads();
   pdl_wait_and_release();
   uint32_t n = 0;
 #pragma unroll
@@ -535,7 +544,7 @@ __global__ void __launch_bounds__(128) cone_kernel(StageParams p, PairList L) {
     if (b == kNoPair) continue;
     float cx, cy, cz;
     cache_position<BF16>(p, L.cache[i], cx, cy, cz);
-    L.shadow[i] = block_cone(p, (int)b, cx, cy, cz, reads);
+    L.shadow[i] = block_cone(p, table, (int)b, cx, cy, cz, reads);
   }
   if constexpr (COUNT) {
     uint32_t a = reads.level0_bytes, b = reads.records, c = reads.texels;
@@ -999,8 +1008,8 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
   if ((e = end(DRV_LK_SCATTER)) != cudaSuccess) return e;
   if (!sur.weights && ((e = skip(DRV_LK_MLP)) != cudaSuccess || (e = wait_voxels()) != cudaSuccess)) return e;
   if ((e = begin(DRV_LK_CONE)) != cudaSuccess) return e;
-  e = count_reads ? launch_grid(cone_kernel<BF16, true>, 128, 0, s, num_sms, cone_ctas, true, p, L)
-                  : launch_grid(cone_kernel<BF16, false>, 128, 0, s, num_sms, cone_ctas, true, p, L);
+  e = count_reads ? launch_grid(cone_kernel<BF16, true>, kConeThreads, 0, s, num_sms, cone_ctas, true, p, L)
+                  : launch_grid(cone_kernel<BF16, false>, kConeThreads, 0, s, num_sms, cone_ctas, true, p, L);
   if (e != cudaSuccess || (e = end(DRV_LK_CONE)) != cudaSuccess || (e = begin(DRV_LK_GATHER)) != cudaSuccess) return e;
   {
     const uint32_t staged = gather_staged_vpls(p.ll, BF16);

@@ -48,11 +48,12 @@ inline VoxelView make_voxel_view(const DrvConfig& cfg, const VoxelInputs& in) {
   v.log2n = L;
   v.max_level = L;
   v.half_mips = cfg.precision == DRV_PRECISION_BF16;
-  v.records = in.records;
-  v.cbias = 0u - tap_index_bias(L);
+  v.inv_n = 1.0f / (float)cfg.voxel_res;
+  v.cbase = (unsigned long long)reinterpret_cast<uintptr_t>(in.corners) - tap_index_bias(L);
   v.record_levels = in.records && in.record_offsets ? in.record_levels : 0;
-  for (int i = 0; i < 16; ++i)
-    v.roff[i] = v.record_levels && i >= 1 && i <= v.record_levels ? in.record_offsets[i] - tap_index_bias(L - i) : 0u;
+  for (int i = 1; i <= v.record_levels && i < 16; ++i)
+    v.rbase[i] = (unsigned long long)reinterpret_cast<uintptr_t>(in.records + in.record_offsets[i]) -
+                 (unsigned long long)tap_index_bias(L - i) * sizeof(uint4);
   return v;
 }
 
@@ -263,19 +264,21 @@ __device__ __forceinline__ bool block_live(const StageParams& p, int b, float cx
   return false;
 }
 
-// Shadowing of block b seen from the cache (the reference's cone); `reads`
-// counts the voxel loads (NoReads: nothing).
-template <class R>
-__device__ __forceinline__ float block_cone(const StageParams& p, int b, float cx, float cy, float cz, R& reads) {
+// Shadowing of block b seen from the cache (the reference's cone); `table`:
+// where the sampler's constants come from; `reads` counts the voxel loads
+// (NoReads: nothing).
+template <class T, class R>
+__device__ __forceinline__ float block_cone(const StageParams& p, const T& table, int b, float cx, float cy, float cz,
+                                            R& reads) {
   const int l = block_light(p, b);
   const float4 c = __ldg(reinterpret_cast<const float4*>(p.ll.lights[l].cones) + (b - p.block_base[l]));
   const float vx = (cx - p.vol_min[0]) * p.inv_extent, vy = (cy - p.vol_min[1]) * p.inv_extent,
               vz = (cz - p.vol_min[2]) * p.inv_extent;
-  return cone_shadow(p.vox, p.voxel_size, p.max_steps, cx, cy, cz, vx, vy, vz, c.x, c.y, c.z, c.w, reads);
+  return cone_shadow(p.vox, table, p.voxel_size, p.max_steps, cx, cy, cz, vx, vy, vz, c.x, c.y, c.z, c.w, reads);
 }
 __device__ __forceinline__ float block_cone(const StageParams& p, int b, float cx, float cy, float cz) {
   NoReads r;
-  return block_cone(p, b, cx, cy, cz, r);
+  return block_cone(p, ViewTable{}, b, cx, cy, cz, r);
 }
 
 // SH gather of one VPL, cacheLightingRSM.comp:255-278. acc (and comp with

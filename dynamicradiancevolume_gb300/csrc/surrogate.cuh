@@ -200,15 +200,15 @@ __device__ __forceinline__ void cone8_features(const VoxelView& v, float inv_ext
   const float inv_len = 1.0f / fmaxf(len, 1e-20f);
   const float Dx = dx * inv_len, Dy = dy * inv_len, Dz = dz * inv_len;
   const float goal = fmaxf(len / voxel_size - 2.0f, 1.0f);  // voxels the cone marches
-  const Coord P = voxel_pos(v, px, py, pz);
   const float lg = __log2f(goal) * 0.125f;
   float transmit = 1.0f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const float d = exp2f(lg * (float)(j + 1));  // marched distance
     const float at = 2.0f + d;                   // from the cache: the march starts 2 voxels out
-    const Coord U{P.x + Dx * at, P.y + Dy * at, P.z + Dz * at};
-    const float s = sample_voxels_at(v, U, __log2f(d * dsr));
+    const float at_s = at * v.inv_n;             // in texture coordinates (exact)
+    const float s = sample_voxels(v, __fmaf_rn(Dx, at_s, px), __fmaf_rn(Dy, at_s, py), __fmaf_rn(Dz, at_s, pz),
+                                  __log2f(d * dsr));
     f[9 + j] = s;
     transmit *= 1.0f - s;
   }
