@@ -780,7 +780,7 @@ drv_status light_caches(DrvContext* ctx, const DrvSpotLight* lights, int32_t n_l
                                   drv::kMaxLightChunks};
   drv_status st = cuda_check(ctx, drv::launch_light_caches(ctx->s(), ctx->cfg, *vol, ll, ctx->counter, ctx->entries,
                                                            ctx->entry_stride, ctx->light_voxels(), scratch,
-                                                           ctx->num_sms),
+                                                           ctx->num_sms, ctx->scratch_words + 1),
                              "light_caches");
   if (st == DRV_OK && ctx->spec_env) st = specular_gather(ctx, ll, vol, frame, nullptr);
   return st;

@@ -283,9 +283,13 @@ cudaError_t launch_build_records(cudaStream_t s, int n, const void* mips, const 
 cudaError_t launch_allocate(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,
                             const float* depth, int w, int h, uint32_t* atlas, void* entries, uint32_t entry_stride,
                             DrvCacheCounter* counter, uint32_t* ticket, uint32_t* err, const float* ndc = nullptr);
+// err: the context's device error word; with it, a stage without indirect
+// shadow runs from VPLs staged in shared memory (whose copy's bounded wait
+// reports there).
 cudaError_t launch_light_caches(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const LightLaunch& ll,
                                 const DrvCacheCounter* counter, void* entries, uint32_t entry_stride,
-                                const VoxelInputs& vox, const LightScratch& scratch, int num_sms);
+                                const VoxelInputs& vox, const LightScratch& scratch, int num_sms,
+                                uint32_t* err = nullptr);
 // The learned visibility surrogate of a light stage: packed weights
 // (nullptr: plain cones), feature set (kFeature*), confidence threshold, the
 // device error word its bounded waits report to, and the timeout test hook

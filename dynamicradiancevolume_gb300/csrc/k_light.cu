@@ -32,8 +32,9 @@
 //     reference's per-light dispatches accumulate).
 //
 // light_kernel, the single-launch form (warp per (cache, chunk) unit, cones
-// traced from a per-warp queue, ticketed chunk reduction), serves the frames
-// without indirect shadow and the allocation-free entry point.
+// traced from a per-warp queue, ticketed chunk reduction), serves the
+// allocation-free entry point and DRV_LIGHT_PATH_SINGLE; unshadowed_kernel the
+// frames without indirect shadow.
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -626,6 +627,64 @@ __device__ __forceinline__ void gather_block_staged(const StageParams& p, const 
   }
 }
 
+// Copies the first `staged` VPLs of the lights' arrays into shared memory (one
+// bulk asynchronous copy per light, issued by thread 0) and their first indices
+// into s_vbase; ends with a CTA barrier. hold (test hook): nothing is copied.
+template <bool BF16>
+__device__ __forceinline__ void stage_vpls_issue(const StageParams& p, unsigned char* s_vpl, uint32_t* s_vbase,
+                                                 uint64_t* s_bar, uint32_t staged, int hold) {
+  if (threadIdx.x == 0) {
+    uint32_t base = 0;
+    for (int l = 0; l < p.ll.n_lights; ++l) {
+      s_vbase[l] = base;
+      base += (uint32_t)p.ll.lights[l].n_vpls;
+    }
+    if (staged) {
+      const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(staged * vpl_bytes<BF16>())
+                   : "memory");
+      for (int l = 0; l < p.ll.n_lights && !hold; ++l) {
+        const uint32_t v0 = s_vbase[l];
+        if (v0 >= staged) break;
+        const uint32_t n = min((uint32_t)p.ll.lights[l].n_vpls, staged - v0);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(s_vpl + (size_t)v0 * vpl_bytes<BF16>())),
+                     "l"(p.ll.lights[l].vpls), "r"(n * vpl_bytes<BF16>()), "r"(bar)
+                     : "memory");
+      }
+    }
+  }
+  __syncthreads();  // offsets written, barrier initialised before anyone waits on it
+}
+
+__device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, unsigned long long limit) {
+  const unsigned long long t0 = clock64();
+  for (;;) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(done)
+        : "r"(bar)
+        : "memory");
+    if (done) return true;
+    if ((unsigned long long)(clock64() - t0) > limit) return false;
+  }
+}
+
+// Waits (bounded) for the copies; false, for the whole CTA, when the wait ran
+// out: the error is latched and the copies were waited for once more, so that
+// the CTA may release its shared memory.
+__device__ __forceinline__ bool stage_vpls_wait(const StageParams& p, uint64_t* s_bar, unsigned long long limit) {
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
+  const bool ok = bar_wait_bounded(bar, limit);
+  if (!__syncthreads_or(!ok)) return true;
+  if (threadIdx.x == 0 && p.err) raise_error(p.err, DRV_DEVERR_TIMEOUT);
+  bar_wait_bounded(bar, limit);
+  return false;
+}
+
 // Warp per gather unit: kGatherChunk pairs of one cache's run (lane j sums
 // the unit's pairs j, j + 32, ... in order), or the whole cache when the list
 // could not hold it (the warp tests every block and traces the live ones'
@@ -653,65 +712,9 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
   constexpr bool KAHAN = BF16;  // FP32 accumulation of BF16-stored results, compensated
   constexpr int NV = NK * 3;
   const int lane = threadIdx.x & 31;
-  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
-  if (threadIdx.x == 0) {
-    uint32_t base = 0;
-    for (int l = 0; l < p.ll.n_lights; ++l) {
-      s_vbase[l] = base;
-      base += (uint32_t)p.ll.lights[l].n_vpls;
-    }
-    if (staged) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(staged * vpl_bytes<BF16>())
-                   : "memory");
-      for (int l = 0; l < p.ll.n_lights && !hold_copy; ++l) {
-        const uint32_t v0 = s_vbase[l];
-        if (v0 >= staged) break;
-        const uint32_t n = min((uint32_t)p.ll.lights[l].n_vpls, staged - v0);
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         (uint32_t)__cvta_generic_to_shared(s_vpl + (size_t)v0 * vpl_bytes<BF16>())),
-                     "l"(p.ll.lights[l].vpls), "r"(n * vpl_bytes<BF16>()), "r"(bar)
-                     : "memory");
-      }
-    }
-  }
-  __syncthreads();  // offsets written, barrier initialised before anyone waits on it
+  stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, hold_copy);
   pdl_wait_and_release();
-  if (staged) {
-    const unsigned long long limit = hold_copy ? kGatherTestWaitCycles : kGatherWaitCycles;
-    bool ok = false;
-    const unsigned long long t0 = clock64();
-    for (;;) {
-      uint32_t done;
-      asm volatile(
-          "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
-          : "=r"(done)
-          : "r"(bar)
-          : "memory");
-      if (done) {
-        ok = true;
-        break;
-      }
-      if ((unsigned long long)(clock64() - t0) > limit) break;
-    }
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0 && p.err) raise_error(p.err, DRV_DEVERR_TIMEOUT);
-      // the copies may still be in flight: wait for them once more (bounded)
-      // before this CTA's shared memory is released
-      const unsigned long long t1 = clock64();
-      for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
-            : "=r"(done)
-            : "r"(bar)
-            : "memory");
-        if (done || (unsigned long long)(clock64() - t1) > limit) break;
-      }
-      return;
-    }
-  }
+  if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kGatherTestWaitCycles : kGatherWaitCycles)) return;
   const uint32_t n_units = L.counters[kGatherUnitsCounter];
   const uint32_t warps = gridDim.x * (THREADS / 32);
   for (uint32_t u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); u < n_units; u += warps) {
@@ -801,6 +804,85 @@ struct FusedParams {
   uint32_t* work;     // unit counter + retired CTAs, zero between launches
 };
 
+// The unit's sums (lane k: coefficient k) into the cache's entry: directly, or
+// through the unit's scratch slot, the last unit of the cache adding the slots
+// in chunk order.
+template <int NK, bool BF16>
+__device__ __forceinline__ void finish_unit(const FusedParams& fp, uint32_t u, uint32_t cache, int lane, float mine) {
+  float* entry = fp.s.entries + (size_t)cache * fp.s.stride_floats;
+  if (fp.n_chunks == 1) {
+    if (lane < NK * 3) add_to_entry<BF16>(entry, lane, mine);
+    return;
+  }
+  if (lane < NK * 3) fp.scratch[(size_t)u * (NK * 3) + lane] = mine;
+  __threadfence();
+  uint32_t last = 0;
+  if (lane == 0) last = atomicAdd(fp.tickets + cache, 1u) == (uint32_t)fp.n_chunks - 1u;
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (last) {
+    __threadfence();
+    if (lane < NK * 3) {
+      const volatile float* sb = fp.scratch + (size_t)cache * fp.n_chunks * (NK * 3);
+      float v = 0.0f;
+      for (int c = 0; c < fp.n_chunks; ++c) v += sb[c * (NK * 3) + lane];
+      add_to_entry<BF16>(entry, lane, v);
+    }
+    if (lane == 0) fp.tickets[cache] = 0u;
+  }
+}
+
+// Without indirect shadow a VPL's pair is a test and, if it faces the cache, 27
+// sums: a warp per (cache, chunk of VPLs) unit, the VPLs staged in shared
+// memory as for the gather, the sums in registers (one 512-thread CTA per SM),
+// whole rounds of 32 VPLs that face away skipped. Bound by issue. 1953
+// caches x 4096 VPLs: 104 us as light_kernel (sums read and written in shared
+// memory for every pair, VPLs from L1) -> about 32 us (the 1280x720 frame 218
+// -> 146 us).
+constexpr int kUnshadowedThreads = 512;
+template <int NK, bool BF16>
+__global__ void __launch_bounds__(kUnshadowedThreads, 1) unshadowed_kernel(FusedParams fp, uint32_t staged) {
+  extern __shared__ __align__(16) unsigned char s_vpl[];
+  __shared__ uint32_t s_vbase[DRV_MAX_LIGHTS];
+  __shared__ __align__(8) uint64_t s_bar;
+  const StageParams& p = fp.s;
+  constexpr bool KAHAN = BF16;
+  constexpr int NV = NK * 3;
+  const int lane = threadIdx.x & 31;
+  stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, 0);
+  const bool ok = !staged || stage_vpls_wait(p, &s_bar, kGatherWaitCycles);
+  const uint32_t n_units = ok ? cache_count(p) * (uint32_t)fp.n_chunks : 0u;
+  for (uint32_t u = next_unit(fp.work, lane); u < n_units; u = next_unit(fp.work, lane)) {
+    const uint32_t cache = u / (uint32_t)fp.n_chunks;
+    const uint32_t lo = (u % (uint32_t)fp.n_chunks) * (uint32_t)fp.chunk_blocks,
+                   hi = min(lo + (uint32_t)fp.chunk_blocks, (uint32_t)p.total_blocks);
+    float cx, cy, cz;
+    cache_position<BF16>(p, cache, cx, cy, cz);
+    float acc[NV], comp[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) acc[q] = comp[q] = 0.0f;
+    for (int l = 0; l < p.ll.n_lights; ++l) {
+      const uint32_t base = s_vbase[l], first = max(lo, base), end = min(hi, base + (uint32_t)p.ll.lights[l].n_vpls);
+      for (uint32_t g0 = first; g0 < end; g0 += 32) {
+        const uint32_t g = min(g0 + (uint32_t)lane, end - 1u);
+        const VplData v = g < staged ? load_vpl<BF16, true>(s_vpl, (int)g)
+                                     : load_vpl<BF16>(p.ll.lights[l].vpls, (int)(g - base));
+        const bool live = g0 + (uint32_t)lane < end && may_contribute(v, cx, cy, cz);
+        if (!__any_sync(0xffffffffu, live)) continue;
+        if (live) {
+          const Transfer t = transfer(v, cx, cy, cz);
+          if (contributes(v, t) && flux_ok(p, v)) accumulate<NK, KAHAN>(p.ev, acc, comp, 1, v, t, 1.0f);
+        }
+      }
+    }
+    float v[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) v[q] = q < NV ? (KAHAN ? __fsub_rn(acc[q], comp[q]) : acc[q]) : 0.0f;
+    const float mine = warp_transpose_reduce<NV <= 16 ? 16 : 32>(v, lane);
+    finish_unit<NK, BF16>(fp, u, cache, lane, mine);
+  }
+  retire_cta(fp.work);
+}
+
 // One warp = one unit (cache, chunk), handed out dynamically; lanes take the
 // chunk's blocks round-robin. Blocks that can contribute go to a per-warp
 // queue traced 32 at a time; partial SH sums live in shared memory (touched
@@ -817,7 +899,6 @@ __global__ void __launch_bounds__(kThreads, 8) light_kernel(FusedParams fp) {
   for (uint32_t u = next_unit(fp.work, lane); u < n_units; u = next_unit(fp.work, lane)) {
     const uint32_t cache = u / (uint32_t)fp.n_chunks;
     const int chunk = (int)(u % (uint32_t)fp.n_chunks);
-    float* entry = p.entries + (size_t)cache * p.stride_floats;
     float cx, cy, cz;
     cache_position<BF16>(p, cache, cx, cy, cz);
     float* acc = s_acc + threadIdx.x;
@@ -875,25 +956,7 @@ __global__ void __launch_bounds__(kThreads, 8) light_kernel(FusedParams fp) {
       for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       if (lane == k) mine = v;
     }
-    if (fp.n_chunks == 1) {
-      if (lane < NK * 3) add_to_entry<BF16>(entry, lane, mine);
-      continue;
-    }
-    if (lane < NK * 3) fp.scratch[(size_t)u * (NK * 3) + lane] = mine;
-    __threadfence();
-    uint32_t last = 0;
-    if (lane == 0) last = atomicAdd(fp.tickets + cache, 1u) == (uint32_t)fp.n_chunks - 1u;
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (last) {
-      __threadfence();
-      if (lane < NK * 3) {
-        const volatile float* sb = fp.scratch + (size_t)cache * fp.n_chunks * (NK * 3);
-        float v = 0.0f;
-        for (int c = 0; c < fp.n_chunks; ++c) v += sb[c * (NK * 3) + lane];
-        add_to_entry<BF16>(entry, lane, v);
-      }
-      if (lane == 0) fp.tickets[cache] = 0u;
-    }
+    finish_unit<NK, BF16>(fp, u, cache, lane, mine);
   }
   retire_cta(fp.work);
 }
@@ -951,6 +1014,23 @@ cudaError_t set_max_smem(const void* kernel, size_t bytes) {
                                                  (int)cudaSharedmemCarveoutMaxShared);
   if (e == cudaSuccess) done.push_back(Done{kernel, dev});
   return e;
+}
+
+// Chunks of whole rounds of 32 VPLs, at most max_chunks per cache, of at least
+// kUnshadowedChunk VPLs (the unshadowed 720p frame: 163 us at 256, 151 at 512,
+// 146 at 1024, 147 at 2048: fewer units leave warps idle, more are reduced more
+// often).
+constexpr int kUnshadowedChunk = 1024;
+template <int NK, bool BF16>
+cudaError_t launch_unshadowed(cudaStream_t s, FusedParams fp, int max_chunks, int num_sms) {
+  const int even = ((fp.s.total_blocks + max_chunks - 1) / max_chunks + 31) & ~31;
+  fp.chunk_blocks = even > kUnshadowedChunk ? even : kUnshadowedChunk;
+  fp.n_chunks = fp.s.total_blocks > 0 ? (fp.s.total_blocks + fp.chunk_blocks - 1) / fp.chunk_blocks : 1;
+  const uint32_t staged = gather_staged_vpls(fp.s.ll, BF16);
+  auto kernel = unshadowed_kernel<NK, BF16>;
+  const cudaError_t e = set_max_smem(reinterpret_cast<const void*>(kernel), kGatherStageBytes);
+  if (e != cudaSuccess) return e;
+  return launch_persistent(kernel, kUnshadowedThreads, (size_t)staged * vpl_bytes<BF16>(), s, num_sms, fp, staged);
 }
 
 // events (optional, 2 x DRV_LK_COUNT): slot k's kernel runs between
@@ -1052,7 +1132,7 @@ int light_chunks(int total_blocks, int max_chunks) {
 
 cudaError_t launch_light_caches(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const LightLaunch& ll,
                                 const DrvCacheCounter* counter, void* entries, uint32_t entry_stride,
-                                const VoxelInputs& vox, const LightScratch& scratch, int num_sms) {
+                                const VoxelInputs& vox, const LightScratch& scratch, int num_sms, uint32_t* err) {
   FusedParams fp;
   fp.s = make_stage_params(cfg, vol, ll, counter, entries, entry_stride, vox);
   fp.n_chunks = light_chunks(fp.s.total_blocks, scratch.max_chunks);
@@ -1061,6 +1141,13 @@ cudaError_t launch_light_caches(cudaStream_t s, const DrvConfig& cfg, const DrvV
   fp.tickets = scratch.tickets;
   fp.work = scratch.work;
   const bool bf16 = cfg.precision == DRV_PRECISION_BF16;
+  if (!cfg.indirect_shadow && err) {
+    fp.s.err = err;
+    return cfg.sh_order == 2 ? (bf16 ? launch_unshadowed<9, true>(s, fp, scratch.max_chunks, num_sms)
+                                     : launch_unshadowed<9, false>(s, fp, scratch.max_chunks, num_sms))
+                             : (bf16 ? launch_unshadowed<4, true>(s, fp, scratch.max_chunks, num_sms)
+                                     : launch_unshadowed<4, false>(s, fp, scratch.max_chunks, num_sms));
+  }
   if (cfg.sh_order == 2)
     return bf16 ? launch_persistent(light_kernel<9, true>, kThreads, 0, s, num_sms, fp)
                 : launch_persistent(light_kernel<9, false>, kThreads, 0, s, num_sms, fp);
