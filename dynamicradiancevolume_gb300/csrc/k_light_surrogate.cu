@@ -3,10 +3,11 @@
 // the split light stage (k_light.cu), on the fifth-generation tensor cores.
 //
 // After the cull has listed the (cache, shadow block) pairs that can
-// contribute, mlp_tc_kernel takes them 128 at a time (one tile per CTA
-// iteration, persistent grid, four CTAs per SM):
+// contribute, mlp_tc_kernel takes them 128 at a time (one tile per group of
+// four warps and iteration, four groups per CTA sharing the weights, persistent
+// grid, two CTAs per SM):
 //  1. each thread computes its pair's 32 input features (surrogate.cuh) and
-//     stores them as BF16 in its row of the CTA's A tile in shared memory;
+//     stores them as BF16 in its row of the group's A tile in shared memory;
 //  2. one thread issues the layer's tcgen05.mma (M = 128 pairs, N = 64
 //     hidden units, K = 16 per instruction, BF16 in, FP32 accumulators in
 //     tensor memory) and commits it to an mbarrier;
@@ -43,11 +44,13 @@
 namespace drv {
 namespace {
 
-constexpr int kThreads = 128;             // one thread per row of the M = 128 tile
+constexpr int kRows = 128;                // one thread per row of the M = 128 tile
+constexpr int kGroups = 4;                // tiles in flight per CTA
+constexpr int kThreads = kRows * kGroups;
 constexpr int kK1 = kMlpIn;               // layer-1 K: 31 features + the constant 1
 constexpr int kKH = kMlpHidden + 16;      // layers 2-4 K: 64 activations, the constant 1, 15 zeros
 constexpr int kN4 = 16;                   // layer-4 N: 2 outputs, padded to the smallest N of an M = 128 MMA
-constexpr int kTmemCols = 64;             // FP32 accumulator columns (N of layers 1-3)
+constexpr int kTmemCols = 64;             // FP32 accumulator columns of a group (N of layers 1-3)
 constexpr float kGeluHalfK = 0.851f;      // 1.702 / 2
 constexpr unsigned long long kWaitCycles = 2000000000ull;  // about one second at 2 GHz
 constexpr unsigned long long kTestWaitCycles = 20000000ull;
@@ -66,13 +69,13 @@ constexpr uint32_t kW2Off = kW1Off + kMlpHidden * kK1 * 2;  // 4096
 constexpr uint32_t kW3Off = kW2Off + kMlpHidden * kKH * 2;  // 14336
 constexpr uint32_t kW4Off = kW3Off + kMlpHidden * kKH * 2;  // 24576
 constexpr uint32_t kWBytes = kW4Off + kN4 * kKH * 2;        // 27136
-constexpr uint32_t kABytes = kThreads * kKH * 2;            // 20480
+constexpr uint32_t kABytes = kRows * kKH * 2;               // 20480
 
 struct __align__(128) TcSmem {
   uint8_t w[kWBytes];
-  uint8_t a[kABytes];
-  uint64_t bar_w;    // the weights' bulk copy
-  uint64_t bar_mma;  // each layer's commit
+  uint8_t a[kGroups][kABytes];
+  uint64_t bar_w;             // the weights' bulk copy
+  uint64_t bar_mma[kGroups];  // each layer's commit
   uint32_t tmem;     // tensor-memory base address (written by tcgen05.alloc)
 };
 
@@ -145,28 +148,22 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
-// Row (TMEM lane) of this thread, 64 consecutive FP32 columns.
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
-  uint32_t r[64];
+// Row (TMEM lane) of this thread, 32 consecutive FP32 columns.
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
+  uint32_t r[32];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,"
-      "%32,%33,%34,%35,%36,%37,%38,%39,%40,%41,%42,%43,%44,%45,%46,%47,"
-      "%48,%49,%50,%51,%52,%53,%54,%55,%56,%57,%58,%59,%60,%61,%62,%63}, [%64];"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]),
-        "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
-        "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]),
-        "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]),
-        "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 __device__ __forceinline__ void tmem_ld2(uint32_t taddr, float& a, float& b) {
@@ -189,10 +186,28 @@ __device__ __forceinline__ uint32_t act_bf16x2(float lo, float hi) {
   return y;
 }
 
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  uint32_t h;
-  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(hi), "f"(lo));
-  return h;
+// A row of the A tile as the features' destination: input k is rounded to BF16
+// and stored where the MMA reads it, so no thread holds its 32 inputs.
+struct FeatureRow {
+  uint8_t* a;
+  int row;
+  struct Input {
+    uint8_t* at;
+    __device__ __forceinline__ void operator=(float x) const { *reinterpret_cast<uint16_t*>(at) = to_bf16(x); }
+  };
+  __device__ __forceinline__ Input operator[](int k) const { return Input{a + kmajor_offset(row, k, kKH)}; }
+};
+
+// The group's barrier (four warps), alone or with an OR over its threads.
+__device__ __forceinline__ void group_sync(int group) { asm volatile("barrier.cta.sync %0, 128;" ::"r"(group + 1) : "memory"); }
+__device__ __forceinline__ bool group_sync_or(int group, bool x) {
+  uint32_t r;
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.u32 q, %2, 0;\nbarrier.cta.red.or.pred p, %1, 128, q;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"(group + 1), "r"((uint32_t)x)
+      : "memory");
+  return r != 0;
 }
 
 // ------------------------------------------------------------ row sources
@@ -207,7 +222,7 @@ struct PairRows {
   __device__ uint32_t rows() const { return min(L.counters[0], L.cap); }
 
   // Writes the row's 32 inputs; false for an empty list slot (inputs 0).
-  __device__ bool features(uint32_t i, float* f) const {
+  __device__ bool features(uint32_t i, const FeatureRow& f) const {
     const uint32_t b = L.block[i];
     if (b == kNoPair) return false;
     float cx, cy, cz;
@@ -249,7 +264,7 @@ struct GivenRows {
   float* out;
 
   __device__ uint32_t rows() const { return n; }
-  __device__ bool features(uint32_t i, float* f) const {
+  __device__ bool features(uint32_t i, const FeatureRow& f) const {
     const float4* x = reinterpret_cast<const float4*>(X + (size_t)i * kMlpIn);
 #pragma unroll
     for (int k = 0; k < kMlpIn / 4; ++k) {
@@ -272,50 +287,59 @@ struct GivenRows {
 };
 
 // ------------------------------------------------------------ the MLP kernel
-// hold_commit: the first layer-1 commit is withheld (its MMAs are not issued
-// either), so that the bounded wait runs out: tests the timeout path.
+// hold_commit: the first layer-1 commit of every group is withheld (its MMAs are
+// not issued either), so that the bounded wait runs out: tests the timeout path.
+//
+// Bound by the latency of the features' voxel loads and of each tile's serial
+// chain of layers, so the SM holds as many tiles as fit: eight groups of four
+// warps (64 registers). 1.8 M pairs, 27 inputs: 295 us with four CTAs of one
+// group and a weight copy each (16 warps per SM), 216 us so, about 195 us with
+// the cone samples' loop rolled (surrogate.cuh).
 template <class Rows>
-__global__ void __launch_bounds__(kThreads, 4) mlp_tc_kernel(Rows src, const uint8_t* __restrict__ wimg,
+__global__ void __launch_bounds__(kThreads, 2) mlp_tc_kernel(Rows src, const uint8_t* __restrict__ wimg,
                                                              uint32_t* err, int hold_commit) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TcSmem& S = *reinterpret_cast<TcSmem*>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int group = threadIdx.x / kRows, tid = threadIdx.x % kRows, warp = tid >> 5;  // within the group
+  uint8_t* A = S.a[group];
+  uint64_t* bar_mma = &S.bar_mma[group];
   const unsigned long long wait_cycles = hold_commit ? kTestWaitCycles : kWaitCycles;
-  if (tid == 0) {
+  if (threadIdx.x == 0) {
     mbar_init(&S.bar_w, 1);
-    mbar_init(&S.bar_mma, 1);
+    for (int g = 0; g < kGroups; ++g) mbar_init(&S.bar_mma[g], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // This row's constant columns of layers 2-4: 1 (BF16 0x3F80), then zeros.
-  *reinterpret_cast<uint4*>(S.a + kmajor_offset(tid, kMlpHidden, kKH)) = make_uint4(0x3F80u, 0u, 0u, 0u);
-  *reinterpret_cast<uint4*>(S.a + kmajor_offset(tid, kMlpHidden + 8, kKH)) = make_uint4(0u, 0u, 0u, 0u);
-  if (warp == 0) {
+  *reinterpret_cast<uint4*>(A + kmajor_offset(tid, kMlpHidden, kKH)) = make_uint4(0x3F80u, 0u, 0u, 0u);
+  *reinterpret_cast<uint4*>(A + kmajor_offset(tid, kMlpHidden + 8, kKH)) = make_uint4(0u, 0u, 0u, 0u);
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem)),
-                 "r"(kTmemCols)
+                 "r"(kTmemCols * kGroups)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = S.tmem;
-  if (tid == 0) bulk_copy_g2s(S.w, wimg, kWBytes, &S.bar_w);
+  const uint32_t tmem_all = S.tmem, tmem = tmem_all + (uint32_t)(kTmemCols * group);
+  if (threadIdx.x == 0) bulk_copy_g2s(S.w, wimg, kWBytes, &S.bar_w);
   bool abort = __syncthreads_or(!mbar_wait_bounded(&S.bar_w, 0, wait_cycles));
 
-  const uint32_t a_addr = smem_u32(S.a), w_addr = smem_u32(S.w);
+  const uint32_t a_addr = smem_u32(A), w_addr = smem_u32(S.w);
   const uint32_t sbo_a = (kKH / 8) * 128;  // 1280
   const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 TMEM lanes
   const uint32_t n_rows = src.rows();
-  const uint32_t n_tiles = (n_rows + kThreads - 1) / kThreads;
+  const uint32_t n_tiles = (n_rows + kRows - 1) / kRows;
   uint32_t phase = 0, evaluated = 0;
   bool held = false;
 
   // One layer: MMAs over k_steps (K = 16 each) of A x W^T into TMEM columns
-  // [0, n), committed; every thread waits for them. False: the wait ran out.
+  // [0, n) of the group, committed; every thread waits for them. False: the
+  // wait ran out.
   auto layer = [&](uint32_t w_off, uint32_t sbo_w, int k_steps, uint32_t idesc) -> bool {
     fence_proxy_async();  // this thread's A-tile stores -> the tensor cores' reads
     tc_fence_before();
-    __syncthreads();
+    group_sync(group);
     if (tid == 0) {
       tc_fence_after();
       if (hold_commit && !held) {
@@ -324,48 +348,41 @@ __global__ void __launch_bounds__(kThreads, 4) mlp_tc_kernel(Rows src, const uin
         for (int ks = 0; ks < k_steps; ++ks)
           mma_bf16(tmem, smem_desc(a_addr + ks * 256, 128, sbo_a), smem_desc(w_addr + w_off + ks * 256, 128, sbo_w),
                    idesc, ks > 0 ? 1u : 0u);
-        mma_commit(&S.bar_mma);
+        mma_commit(bar_mma);
       }
     }
-    const bool ok = mbar_wait_bounded(&S.bar_mma, phase, wait_cycles);
+    const bool ok = mbar_wait_bounded(bar_mma, phase, wait_cycles);
     phase ^= 1u;
     tc_fence_after();
-    return !__syncthreads_or(!ok);
+    const bool all = !group_sync_or(group, !ok);
+    __syncwarp();  // the accumulators' reads below are warp-wide
+    return all;
   };
   // Accumulators -> activations -> this thread's row of the A tile.
   auto activate = [&]() {
-    float v[64];
-    tmem_ld64(t_row, v);
 #pragma unroll
-    for (int c = 0; c < kMlpHidden / 8; ++c) {
-      uint4 q;
-      q.x = act_bf16x2(v[8 * c + 0], v[8 * c + 1]);
-      q.y = act_bf16x2(v[8 * c + 2], v[8 * c + 3]);
-      q.z = act_bf16x2(v[8 * c + 4], v[8 * c + 5]);
-      q.w = act_bf16x2(v[8 * c + 6], v[8 * c + 7]);
-      *reinterpret_cast<uint4*>(S.a + kmajor_offset(tid, 8 * c, kKH)) = q;
+    for (int h = 0; h < 2; ++h) {
+      float v[32];
+      tmem_ld32(t_row + 32 * h, v);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        uint4 q;
+        q.x = act_bf16x2(v[8 * c + 0], v[8 * c + 1]);
+        q.y = act_bf16x2(v[8 * c + 2], v[8 * c + 3]);
+        q.z = act_bf16x2(v[8 * c + 4], v[8 * c + 5]);
+        q.w = act_bf16x2(v[8 * c + 6], v[8 * c + 7]);
+        *reinterpret_cast<uint4*>(A + kmajor_offset(tid, 32 * h + 8 * c, kKH)) = q;
+      }
     }
   };
 
-  for (uint32_t tile = blockIdx.x; tile < n_tiles && !abort; tile += gridDim.x) {
-    const uint32_t row = tile * kThreads + tid;
-    bool valid = false;
-    {
-      float f[kMlpIn];
-      if (row < n_rows) valid = src.features(row, f);
-      if (!valid) {
+  for (uint32_t tile = blockIdx.x * kGroups + group; tile < n_tiles && !abort; tile += gridDim.x * kGroups) {
+    const uint32_t row = tile * kRows + tid;
+    const bool valid = row < n_rows && src.features(row, FeatureRow{A, tid});
+    if (!valid) {
 #pragma unroll
-        for (int k = 0; k < kMlpIn; ++k) f[k] = 0.0f;
-      }
-#pragma unroll
-      for (int c = 0; c < kMlpIn / 8; ++c) {
-        uint4 q;
-        q.x = pack2(f[8 * c + 0], f[8 * c + 1]);
-        q.y = pack2(f[8 * c + 2], f[8 * c + 3]);
-        q.z = pack2(f[8 * c + 4], f[8 * c + 5]);
-        q.w = pack2(f[8 * c + 6], f[8 * c + 7]);
-        *reinterpret_cast<uint4*>(S.a + kmajor_offset(tid, 8 * c, kKH)) = q;
-      }
+      for (int c = 0; c < kMlpIn / 8; ++c)
+        *reinterpret_cast<uint4*>(A + kmajor_offset(tid, 8 * c, kKH)) = make_uint4(0u, 0u, 0u, 0u);
     }
     if (!(abort = !layer(kW1Off, (kK1 / 8) * 128, kK1 / 16, instr_desc(kMlpHidden)))) activate();
     if (!abort && !(abort = !layer(kW2Off, sbo_a, kKH / 16, instr_desc(kMlpHidden)))) activate();
@@ -373,23 +390,24 @@ __global__ void __launch_bounds__(kThreads, 4) mlp_tc_kernel(Rows src, const uin
     if (!abort && !(abort = !layer(kW4Off, sbo_a, kKH / 16, instr_desc(kN4)))) {
       float o_vis, o_conf;
       tmem_ld2(t_row, o_vis, o_conf);
-      src.finish(row, valid && row < n_rows, o_vis, o_conf, evaluated);
+      src.finish(row, valid, o_vis, o_conf, evaluated);
     }
   }
   if (abort) {
     if (tid == 0) raise_error(err, DRV_DEVERR_TIMEOUT);
-    // What this CTA issued may still be in flight: wait for it once more
+    // What this group issued may still be in flight: wait for it once more
     // (bounded) before the tensor memory and shared memory are released.
     mbar_wait_bounded(&S.bar_w, 0, wait_cycles);
-    if (phase) mbar_wait_bounded(&S.bar_mma, phase ^ 1u, wait_cycles);
+    if (phase) mbar_wait_bounded(bar_mma, phase ^ 1u, wait_cycles);
   } else {
     src.done(evaluated);
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_all), "r"(kTmemCols * kGroups)
+                 : "memory");
 }
 
 // FP32 master parameters -> the packed BF16 B-operand image (folded biases
@@ -441,18 +459,17 @@ cudaError_t launch_tc(cudaStream_t s, const Rows& rows, uint32_t n_rows, const v
     if (dev >= 64 || !((done >> dev) & 1u)) {
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
-      // Four CTAs of ~47 KB per SM need the largest shared-memory carveout.
+      // Two CTAs of ~107 KB per SM need the largest shared-memory carveout.
       e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                (int)cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return e;
       if (dev < 64) done |= 1ull << dev;
     }
   }
-  // Four CTAs per SM (__launch_bounds__; 4 x 64 of the SM's 512 tensor-memory
-  // columns): the CTAs of one SM overlap each other's MMA round trips.
-  const int per_sm = 4;
-  const uint32_t tiles = (n_rows + kThreads - 1) / kThreads;
-  const uint32_t grid = tiles == 0 ? 1u : (tiles < (uint32_t)(num_sms * per_sm) ? tiles : (uint32_t)(num_sms * per_sm));
+  // Two CTAs per SM (__launch_bounds__; 2 x 256 of the SM's 512 tensor-memory
+  // columns): the groups of one SM overlap each other's loads and MMA round trips.
+  const uint32_t ctas = (n_rows + kThreads - 1) / kThreads, most = (uint32_t)num_sms * 2u;
+  const uint32_t grid = ctas == 0 ? 1u : (ctas < most ? ctas : most);
   kernel<<<grid, kThreads, smem, s>>>(rows, static_cast<const uint8_t*>(weights), err, hold_commit);
   return cudaGetLastError();
 }

@@ -80,10 +80,11 @@ __device__ __forceinline__ float cone_reach(float goal, float dsr, int max_steps
 //   traces, 17 aperture, 18 length, 19-21 direction, 22-25 the cone's own
 //   first four samples (same positions and LOD as cacheLightingRSM.comp:
 //   211-225), 26 their composited occlusion.
+template <class F>
 __device__ __forceinline__ void surrogate_features(const VoxelView& v, float inv_extent, const float vol_min[3],
                                                    float voxel_size, int max_steps, float cx, float cy, float cz,
                                                    float tx, float ty, float tz, float nx, float ny, float nz,
-                                                   float dsr, float* f) {
+                                                   float dsr, F&& f) {
   const float px = (cx - vol_min[0]) * inv_extent, py = (cy - vol_min[1]) * inv_extent,
               pz = (cz - vol_min[2]) * inv_extent;
   const float qx = (tx - vol_min[0]) * inv_extent, qy = (ty - vol_min[1]) * inv_extent,
@@ -122,7 +123,9 @@ __device__ __forceinline__ void surrogate_features(const VoxelView& v, float inv
     float ux = px + sx * 2.0f, uy = py + sy * 2.0f, uz = pz + sz * 2.0f;
     float step = 1.0f, dist = 0.0f, transmit = 1.0f;
     const float k = 2.0f / (1.0f - dsr);
-#pragma unroll
+// Rolled: four copies of the sampler overflow the instruction cache (frame of
+// 1.8 M pairs 432 -> 412 us).
+#pragma unroll 1
     for (int s = 0; s < 4; ++s) {
       ux += sx * step;
       uy += sy * step;
@@ -146,9 +149,10 @@ __device__ __forceinline__ void surrogate_features(const VoxelView& v, float inv
 // volume coordinates, 6-8 the VPL normal, 9-16 eight trilinear opacity
 // samples of mip level 3 at the midpoints of eight equal parts of the
 // segment from the cache to the target; 31 the constant 1.
+template <class F>
 __device__ __forceinline__ void segment_features(const VoxelView& v, float inv_extent, const float vol_min[3],
                                                  float cx, float cy, float cz, float tx, float ty, float tz, float nx,
-                                                 float ny, float nz, float* f) {
+                                                 float ny, float nz, F&& f) {
   const float px = (cx - vol_min[0]) * inv_extent, py = (cy - vol_min[1]) * inv_extent,
               pz = (cz - vol_min[2]) * inv_extent;
   const float qx = (tx - vol_min[0]) * inv_extent, qy = (ty - vol_min[1]) * inv_extent,
@@ -179,9 +183,10 @@ __device__ __forceinline__ void segment_features(const VoxelView& v, float inv_e
 // the cone's steps grow), 17 their composited occlusion 1 - prod(1 - s),
 // 18 the aperture (x 8), 19 the march length in voxels (/ 64), 20-22 the
 // direction; 31 the constant 1.
+template <class F>
 __device__ __forceinline__ void cone8_features(const VoxelView& v, float inv_extent, const float vol_min[3],
                                                float voxel_size, float cx, float cy, float cz, float tx, float ty,
-                                               float tz, float nx, float ny, float nz, float dsr, float* f) {
+                                               float tz, float nx, float ny, float nz, float dsr, F&& f) {
   const float px = (cx - vol_min[0]) * inv_extent, py = (cy - vol_min[1]) * inv_extent,
               pz = (cz - vol_min[2]) * inv_extent;
   const float qx = (tx - vol_min[0]) * inv_extent, qy = (ty - vol_min[1]) * inv_extent,
@@ -223,12 +228,13 @@ __device__ __forceinline__ void cone8_features(const VoxelView& v, float inv_ext
   f[kOneInput] = 1.0f;
 }
 
-// Features of a pair in feature set FS.
-template <int FS>
+// Features of a pair in feature set FS into f[0..31] (floats, or inputs that
+// convert what is assigned).
+template <int FS, class F>
 __device__ __forceinline__ void pair_features(const VoxelView& v, float inv_extent, const float vol_min[3],
                                               float voxel_size, int max_steps, float cx, float cy, float cz,
                                               float tx, float ty, float tz, float nx, float ny, float nz, float dsr,
-                                              float* f) {
+                                              F&& f) {
   if (FS == kFeatureSegment8)
     segment_features(v, inv_extent, vol_min, cx, cy, cz, tx, ty, tz, nx, ny, nz, f);
   else if (FS == kFeatureCone8)
