@@ -69,6 +69,7 @@ void release(Context* c) {
     cudaFree(c->vpls[l]);
     cudaFree(c->cones[l]);
     cudaFree(c->vpl_records[l]);
+    cudaFree(c->cone_steps[l]);
   }
   cudaFree(c->d_boxes);
   cudaFreeHost(c->h_boxes);
@@ -316,6 +317,7 @@ drv_status drv_create(const DrvConfig* cfg, DrvContext** out) {
     if ((e = cudaMalloc(&c->vpls[l], (size_t)R * R * sizeof(DrvVPL))) != cudaSuccess) return bail(e);
     if ((e = cudaMalloc(&c->cones[l], (size_t)R * R * sizeof(DrvShadowCone))) != cudaSuccess) return bail(e);
     if ((e = cudaMalloc(&c->vpl_records[l], (size_t)R * R * sizeof(float4))) != cudaSuccess) return bail(e);
+    if ((e = cudaMalloc(&c->cone_steps[l], (size_t)R * R * sizeof(float4))) != cudaSuccess) return bail(e);
   }
   if ((e = cudaMalloc(&c->sur_weights, drv::surrogate_weights_bytes())) != cudaSuccess) return bail(e);
   // Pair list of the split light stage: room for 256 contributing shadow
@@ -595,7 +597,7 @@ drv_status drv_extract_vpls(DrvContext* ctx, int32_t li, const DrvSpotLight* L) 
   DRV_TRY_CUDA(ctx, drv::launch_extract_vpls(ctx->s(), *L, R, ch.flux[read_lod], ch.normal[read_lod], ch.dls[read_lod],
                                              ch.half(read_lod), ch.dls[shadow_level], ch.half(shadow_level),
                                              ctx->vpls[li], ctx->cones[li], ctx->cfg.precision,
-                                             ctx->vpl_records[li]));
+                                             ctx->vpl_records[li], ctx->cone_steps[li]));
   ctx->n_vpls[li] = R * R;
   ctx->interval[li] = L->indirect_shadow_sample_interval;
   ctx->n_cones[li] = (R * R + L->indirect_shadow_sample_interval - 1) / L->indirect_shadow_sample_interval;
@@ -702,6 +704,7 @@ drv_status light_caches(DrvContext* ctx, const DrvSpotLight* lights, int32_t n_l
     ll.lights[l].n_vpls = ctx->n_vpls[l];
     ll.lights[l].interval = ctx->interval[l];
     ll.lights[l].records = ctx->vpl_records[l];
+    ll.lights[l].steps = ctx->cone_steps[l];
   }
   const bool surrogate = ctx->cfg.visibility == DRV_VISIBILITY_SURROGATE && ctx->cfg.indirect_shadow;
   if (surrogate && !ctx->sur_ready)

@@ -269,4 +269,17 @@ __device__ __forceinline__ float4 make_cull_record(float nx, float ny, float nz,
   return make_float4(nx, ny, nz, flux ? -(nx * px + ny * py + nz * pz) + kCullRecordEps * (1.0f + pm) : -INFINITY);
 }
 
+// What the ordering of the shadow cones needs of a block's aperture
+// (k_light.cu, cone_class): cone_shadow steps by max(1, g * dist) with
+// g = 2 dsr / (1 - dsr): unit steps up to the distance m = floor(1 / g), then
+// the distance grows by 1 + g per step. {m, 1 / log2(1 + g), log2 m, the first
+// step whose radius passes one voxel}.
+__device__ __forceinline__ float4 make_cone_steps(float dsr) {
+  const float g = 2.0f * dsr / (1.0f - dsr);
+  const float m = g > 0.0f ? fmaxf(1.0f, floorf(1.0f / g)) : 3.0e38f;
+  const float inv = 1.0f / __log2f(1.0f + g), lm = __log2f(m);
+  const float wide = 1.0f / dsr;  // distance at which the radius is one voxel
+  return make_float4(m, inv, lm, dsr > 0.0f ? (wide <= m ? wide : m + (__log2f(wide) - lm) * inv) : 3.0e38f);
+}
+
 }  // namespace drv

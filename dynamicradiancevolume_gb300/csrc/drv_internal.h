@@ -52,6 +52,7 @@ struct LightArgs {
   int n_vpls;
   int interval;  // IndirectShadowComputationSampleInterval
   const float4* records = nullptr;  // the cull's VPL plane records (make_cull_record), or none
+  const float4* steps = nullptr;    // per shadow block, for the ordering of its cones (make_cone_steps)
 };
 
 struct LightLaunch {
@@ -213,6 +214,7 @@ struct Context {
   void* vpls[DRV_MAX_LIGHTS] = {};  // DrvVPL or DrvVPLBF16 per cfg.precision
   DrvShadowCone* cones[DRV_MAX_LIGHTS] = {};
   float4* vpl_records[DRV_MAX_LIGHTS] = {};  // the cull's plane record of every VPL (written by the extraction)
+  float4* cone_steps[DRV_MAX_LIGHTS] = {};   // make_cone_steps of every shadow block (written by the extraction)
   int n_vpls[DRV_MAX_LIGHTS] = {};
   int n_cones[DRV_MAX_LIGHTS] = {};
   int interval[DRV_MAX_LIGHTS] = {};
@@ -265,7 +267,7 @@ cudaError_t launch_rsm_chain(cudaStream_t s, int res, int passes, const void* fl
                              const void* dls, int src_half, float* const* fo, int16_t* const* no, float* const* dlo);
 cudaError_t launch_extract_vpls(cudaStream_t s, const DrvSpotLight& L, int res, const void* flux, const int16_t* nrm,
                                 const void* dls, int read_half, const void* dls_shadow, int shadow_half, void* vpls,
-                                DrvShadowCone* cones, int precision, float4* records);
+                                DrvShadowCone* cones, int precision, float4* records, float4* steps);
 cudaError_t launch_voxelize(cudaStream_t s, const DrvBox* boxes, int n_boxes, const DrvVolumeInfo& vol, int n,
                             uint32_t* bits);
 cudaError_t launch_voxelize_triangles(cudaStream_t s, const float* positions, int n_vertices, const uint32_t* indices,

@@ -413,23 +413,14 @@ __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StagePara
 // Cone class of a pair: about how many steps its cone marches when nothing
 // occludes it, in buckets of 4, and at which step, if any, its radius passes
 // one voxel (its samples move to mip levels): never, after step 16, after
-// step 8, or earlier. cone_shadow steps by max(1, g * dist) with
-// g = 2 dsr / (1 - dsr): unit steps up to dist = 1 / g, then the distance
-// grows by the factor 1 + g per step, until it reaches the goal. Classes
-// only order the cones; results do not depend on them.
-__device__ __forceinline__ float cone_steps_to(float dist, float g, float m) {
-  // steps until the marched distance reaches `dist`
-  return dist <= m ? ceilf(dist) : m + ceilf(__log2f(dist / m) / __log2f(1.0f + g));
-}
-
-__device__ __forceinline__ int cone_class(float light_dist, float voxel_size, float dsr, int max_steps) {
-  const float goal = fmaxf(light_dist / voxel_size - 2.0f, 1.0f);
-  const float g = 2.0f * dsr / (1.0f - dsr);
-  const float m = g > 0.0f ? fmaxf(1.0f, floorf(1.0f / g)) : 3.0e38f;  // last unit step
-  const float n = fminf(cone_steps_to(goal, g, m), (float)max_steps);
-  const float n_mip = dsr > 0.0f ? cone_steps_to(1.0f / dsr, g, m) : 3.0e38f;  // first step with radius > 1
+// step 8, or earlier. What depends on the block alone comes from the extraction
+// (st: make_cone_steps); per pair the distance and one logarithm are left.
+// Classes only order the cones; results do not depend on them.
+__device__ __forceinline__ int cone_class(float light_dist, float inv_voxel, const float4 st, float max_steps) {
+  const float goal = fmaxf(light_dist * inv_voxel - 2.0f, 1.0f);
+  const float n = fminf(goal <= st.x ? goal : st.x + (__log2f(goal) - st.z) * st.y, max_steps);
   const int len = min(max((int)n - 1, 0) >> 2, 7);
-  const int mip = n_mip > n ? 0 : (n_mip > 16.0f ? 1 : (n_mip > 8.0f ? 2 : 3));
+  const int mip = st.w > n ? 0 : (st.w > 16.0f ? 1 : (st.w > 8.0f ? 2 : 3));
   return mip * 8 + len;
 }
 
@@ -437,7 +428,11 @@ constexpr int kClassThreads = 256;
 
 // Thread per listed pair: its cone class; class totals in counters[8 + c].
 // MARKED: only the pairs the surrogate left unconfident (cls 0) get a class;
-// the others keep 0xFF and are neither ordered nor traced.
+// the others keep 0xFF and are neither ordered nor traced. Bound by the
+// latency of its dependent loads; 3.9 M pairs: 37 -> 24 us (230 instructions a
+// pair with the cone's step rule evaluated in full). Two or four pairs per
+// thread, their loads together, are slower (614 and 629 us for the frame against
+// 610: fewer warps).
 template <bool BF16, bool MARKED>
 __global__ void __launch_bounds__(kClassThreads) classify_kernel(StageParams p, PairList L) {
   pdl_wait_and_release();
@@ -445,16 +440,19 @@ __global__ void __launch_bounds__(kClassThreads) classify_kernel(StageParams p, 
   if (threadIdx.x < kConeClasses) s_hist[threadIdx.x] = 0u;
   __syncthreads();
   const uint32_t n = min(L.counters[0], L.cap);
+  const float inv_voxel = 1.0f / p.voxel_size, max_steps = (float)p.max_steps;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t b = L.block[i];
     uint8_t c = 0xFF;
     if (b != kNoPair && (!MARKED || L.cls[i] != 0xFF)) {
       float cx, cy, cz;
       cache_position<BF16>(p, L.cache[i], cx, cy, cz);
-      const int l = block_light(p, (int)b);
-      const float4 cone = __ldg(reinterpret_cast<const float4*>(p.ll.lights[l].cones) + (b - p.block_base[l]));
+      const int l = block_light(p, (int)b), lb = (int)b - p.block_base[l];
+      const float4 cone = __ldg(reinterpret_cast<const float4*>(p.ll.lights[l].cones) + lb);
+      const float4 st = __ldg(p.ll.lights[l].steps + lb);
       const float tx = cone.x - cx, ty = cone.y - cy, tz = cone.z - cz;
-      c = (uint8_t)cone_class(sqrtf(tx * tx + ty * ty + tz * tz), p.voxel_size, cone.w, p.max_steps);
+      const float d2 = tx * tx + ty * ty + tz * tz;
+      c = (uint8_t)cone_class(d2 * rsqrtf(fmaxf(d2, 1e-30f)), inv_voxel, st, max_steps);
       atomicAdd(&s_hist[c], 1u);
     }
     L.cls[i] = c;
@@ -463,11 +461,16 @@ __global__ void __launch_bounds__(kClassThreads) classify_kernel(StageParams p, 
   if (threadIdx.x < kConeClasses && s_hist[threadIdx.x]) atomicAdd(L.counters + 8 + threadIdx.x, s_hist[threadIdx.x]);
 }
 
-constexpr int kScatterTile = 4 * kClassThreads;
+constexpr int kScatterPerThread = 8;
+constexpr int kScatterTile = kScatterPerThread * kClassThreads;
 
-// CTA per tile of kScatterTile pairs (4 per thread): each pair's index goes
-// to its class's region of L.order (regions in class order); a CTA reserves
-// its share of each region with one atomic per class.
+// CTA per tile of kScatterTile pairs: each pair's index goes to its class's
+// region of L.order (regions in class order); a CTA reserves its share of each
+// region with one atomic per class. A warp's pairs of one class (consecutive
+// pairs mostly are) take one shared-memory atomic together and keep their
+// order, so that neighbouring cones stay neighbours (the cone pass of 5.5 M pairs 402 ->
+// 393 us). 8 pairs per thread; 4 measure the same, 16 are slower (610, 611 and
+// 615 us for the 1080p frame).
 __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
   pdl_wait_and_release();
   __shared__ uint32_t s_region[kConeClasses], s_hist[kConeClasses], s_pos[kConeClasses];
@@ -484,16 +487,24 @@ __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
     }
     s_region[threadIdx.x] = incl - total;
   }
+  const int lane = threadIdx.x & 31;
   for (uint32_t t0 = blockIdx.x * kScatterTile; t0 < n; t0 += gridDim.x * kScatterTile) {
     if (threadIdx.x < kConeClasses) s_hist[threadIdx.x] = 0u;
-    __syncthreads();
-    uint8_t c[4];
-    uint32_t rank[4];
+    uint8_t c[kScatterPerThread];
+    uint32_t rank[kScatterPerThread];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < kScatterPerThread; ++j) {
       const uint32_t i = t0 + j * kClassThreads + threadIdx.x;
       c[j] = i < n ? L.cls[i] : (uint8_t)0xFF;
-      rank[j] = c[j] != 0xFF ? atomicAdd(&s_hist[c[j]], 1u) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kScatterPerThread; ++j) {
+      const uint32_t peers = __match_any_sync(0xffffffffu, (uint32_t)c[j]);
+      const int first = __ffs(peers) - 1;
+      uint32_t base = 0;
+      if (lane == first && c[j] != 0xFF) base = atomicAdd(&s_hist[c[j]], (uint32_t)__popc(peers));
+      rank[j] = __shfl_sync(0xffffffffu, base, first) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
     }
     __syncthreads();
     if (threadIdx.x < kConeClasses) {
@@ -502,7 +513,7 @@ __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < kScatterPerThread; ++j)
       if (c[j] != 0xFF) L.order[s_pos[c[j]] + rank[j]] = t0 + j * kClassThreads + threadIdx.x;
     __syncthreads();
   }

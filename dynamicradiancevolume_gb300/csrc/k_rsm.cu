@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) extract_kernel(DrvSpotLight L, int R, con
                                                       int read_half, const void* __restrict__ dls_shadow,
                                                       int shadow_half, void* __restrict__ vpls_out,
                                                       DrvShadowCone* __restrict__ cones,
-                                                      float4* __restrict__ records) {
+                                                      float4* __restrict__ records, float4* __restrict__ steps) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   int n = R * R;
   if (i >= n) return;
@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(256) extract_kernel(DrvSpotLight L, int R, con
     float var = fmaxf(0.0f, dd1 - dd0 * dd0);  // clamped: rounding can push it below 0
     float dsr = fmaxf(L.indirect_shadow_super_val_width, sqrtf(var) * 2.0f / dd0);
     cones[i] = DrvShadowCone{{avg.x, avg.y, avg.z}, dsr};
+    steps[i] = make_cone_steps(dsr);
   }
 }
 
@@ -234,14 +235,14 @@ cudaError_t launch_rsm_chain(cudaStream_t s, int res, int passes, const void* fl
 
 cudaError_t launch_extract_vpls(cudaStream_t s, const DrvSpotLight& L, int res, const void* flux, const int16_t* nrm,
                                 const void* dls, int read_half, const void* dls_shadow, int shadow_half, void* vpls,
-                                DrvShadowCone* cones, int precision, float4* records) {
+                                DrvShadowCone* cones, int precision, float4* records, float4* steps) {
   int n = res * res;
   if (precision == DRV_PRECISION_BF16)
     extract_kernel<true><<<(n + 255) / 256, 256, 0, s>>>(L, res, flux, nrm, dls, read_half, dls_shadow, shadow_half,
-                                                         vpls, cones, records);
+                                                         vpls, cones, records, steps);
   else
     extract_kernel<false><<<(n + 255) / 256, 256, 0, s>>>(L, res, flux, nrm, dls, read_half, dls_shadow, shadow_half,
-                                                          vpls, cones, records);
+                                                          vpls, cones, records, steps);
   return cudaGetLastError();
 }
 
