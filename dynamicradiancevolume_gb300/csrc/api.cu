@@ -48,6 +48,7 @@ void release(Context* c) {
   cudaFree(c->mips);
   cudaFree(c->vox_corners);
   cudaFree(c->vox_records);
+  cudaFree(c->vox_wide);
   cudaFree(c->ndc);
   cudaFree(c->srgb);
   cudaFree(c->raster_mem);
@@ -301,6 +302,8 @@ drv_status drv_create(const DrvConfig* cfg, DrvContext** out) {
   }
   c->record_offset[c->record_levels + 1] = records;
   if (records && (e = cudaMalloc(&c->vox_records, (size_t)records * 16)) != cudaSuccess) return bail(e);
+  const size_t wide = drv::wide_record_bytes(c->n_voxel_levels, c->record_levels);
+  if (wide && (e = cudaMalloc(&c->vox_wide, wide)) != cudaSuccess) return bail(e);
 
   // The single-launch light stage's scratch, where frames need it from the
   // start (no indirect shadow); otherwise on first use (ensure_single_scratch).
@@ -644,7 +647,8 @@ drv_status drv_build_opacity_mips(DrvContext* ctx) {
   if (st == DRV_OK)
     st = cuda_check(ctx,
                     drv::launch_build_records(s, ctx->cfg.voxel_res, ctx->mips, ctx->mip_offset, ctx->cfg.precision,
-                                              ctx->vox_records, ctx->record_offset, ctx->record_levels),
+                                              ctx->vox_records, ctx->record_offset, ctx->record_levels, ctx->vox_wide,
+                                              ctx->n_voxel_levels),
                     "build_records");
   DRV_TRY_CUDA(ctx, cudaEventRecord(ctx->join_ev[2], ctx->side[2]));
   DRV_TRY_CUDA(ctx, cudaStreamWaitEvent(s, ctx->join_ev[2], 0));

@@ -68,7 +68,18 @@ struct VoxelInputs {
   const uint4* records = nullptr;       // corner-packed mip records of levels 1..record_levels (optional)
   const uint32_t* record_offsets = nullptr;  // record offset of each level (index 1..record_levels + 1)
   int record_levels = 0;
+  const void* wide_records = nullptr;   // FP32 records of levels record_levels + 1..L, back to back (optional)
 };
+
+// An FP32 mip record (the levels whose texels FP16 does not hold exactly).
+constexpr int kWideRecordBytes = 32;
+// Bytes of all FP32 records of a pyramid with levels 1..n_levels - 1 of which
+// record_levels have FP16 records.
+inline size_t wide_record_bytes(int n_levels, int record_levels) {
+  size_t b = 0;
+  for (int l = record_levels + 1; l < n_levels; ++l) b += (size_t)kWideRecordBytes << (3 * (n_levels - 1 - l));
+  return b;
+}
 
 // Levels that get corner-packed FP16 mip records: every level with BF16
 // precision (FP16 texels); levels 1..3 with FP32 precision, whose texels
@@ -194,6 +205,7 @@ struct Context {
   size_t mip_offset[kMaxVoxelLevels] = {};
   uint4* vox_records = nullptr;  // corner-packed mip records (voxel_sample.cuh)
   uint32_t record_offset[kMaxVoxelLevels + 1] = {};
+  void* vox_wide = nullptr;  // FP32 records of the levels above (FP32 precision)
   int record_levels = 0;
   // The voxel inputs of the light stage: without the mip records when
   // DrvTuning.plain_voxel_reads asks for it.
@@ -202,11 +214,12 @@ struct Context {
     if (tuning.plain_voxel_reads) {
       v.records = nullptr;
       v.record_levels = 0;
+      v.wide_records = nullptr;
     }
     return v;
   }
   VoxelInputs voxels() const {
-    return VoxelInputs{vox_corners, mips, mip_offset, vox_records, record_offset, record_levels};
+    return VoxelInputs{vox_corners, mips, mip_offset, vox_records, record_offset, record_levels, vox_wide};
   }
   int n_voxel_levels = 0;
   // RSM + VPLs per light.
@@ -281,7 +294,8 @@ cudaError_t launch_build_mips(cudaStream_t s, int n, const uint32_t* bits, void*
                               int n_levels, int precision, uint32_t* ticket);
 cudaError_t launch_build_corners(cudaStream_t s, int n, const uint32_t* bits, uint8_t* corners);
 cudaError_t launch_build_records(cudaStream_t s, int n, const void* mips, const size_t* mip_offsets, int precision,
-                                 uint4* records, const uint32_t* record_offsets, int record_levels);
+                                 uint4* records, const uint32_t* record_offsets, int record_levels, void* wide,
+                                 int n_levels);
 cudaError_t launch_allocate(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,
                             const float* depth, int w, int h, uint32_t* atlas, void* entries, uint32_t entry_stride,
                             DrvCacheCounter* counter, uint32_t* ticket, uint32_t* err, const float* ndc = nullptr);

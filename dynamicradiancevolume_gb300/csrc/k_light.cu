@@ -530,10 +530,11 @@ __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
 // warp instructions). Six CTAs per SM (40 registers) against five: 633 / 642 us
 // for the frame; 128-thread CTAs leave the tables less L1 (651 against 642).
 constexpr int kConeThreads = 256;
-template <bool BF16, bool COUNT = false>
+// PLAIN: some levels have no records (DrvTuning.plain_voxel_reads).
+template <bool BF16, bool COUNT, bool PLAIN>
 __global__ void __launch_bounds__(kConeThreads, 6) cone_kernel(StageParams p, PairList L) {
   __shared__ SharedTableStorage s_table;
-  const SharedTable table = fill_table(s_table, p.vox);
+  const SharedTable<PLAIN> table = fill_table<PLAIN>(s_table, p.vox);
   __syncthreads();
   pdl_wait_and_release();
   uint32_t n = 0;
@@ -1099,8 +1100,12 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
   if ((e = end(DRV_LK_SCATTER)) != cudaSuccess) return e;
   if (!sur.weights && ((e = skip(DRV_LK_MLP)) != cudaSuccess || (e = wait_voxels()) != cudaSuccess)) return e;
   if ((e = begin(DRV_LK_CONE)) != cudaSuccess) return e;
-  e = count_reads ? launch_grid(cone_kernel<BF16, true>, kConeThreads, 0, s, num_sms, cone_ctas, true, p, L)
-                  : launch_grid(cone_kernel<BF16, false>, kConeThreads, 0, s, num_sms, cone_ctas, true, p, L);
+  {
+    const bool plain = p.vox.wide_levels < p.vox.max_level;
+    auto kernel = count_reads ? (plain ? cone_kernel<BF16, true, true> : cone_kernel<BF16, true, false>)
+                              : (plain ? cone_kernel<BF16, false, true> : cone_kernel<BF16, false, false>);
+    e = launch_grid(kernel, kConeThreads, 0, s, num_sms, cone_ctas, true, p, L);
+  }
   if (e != cudaSuccess || (e = end(DRV_LK_CONE)) != cudaSuccess || (e = begin(DRV_LK_GATHER)) != cudaSuccess) return e;
   {
     const uint32_t staged = gather_staged_vpls(p.ll, BF16);

@@ -493,10 +493,12 @@ __global__ void __launch_bounds__(256) corners_kernel(int N, int log2n, const ui
 // the record pairs (x0, x0 + 1) of a warp fill contiguous rows). Records
 // hold FP16 texels: a copy with BF16 precision; with FP32 precision the
 // records cover levels 1..3, whose texels k / 8^l (8^l <= 512) FP16 holds
-// exactly.
+// exactly, and the levels above get FP32 records (the same slots, 32 bytes), in
+// an array of their own.
 struct RecordLevels {
-  uint32_t blocks;  // 2x2x2 record blocks of levels 1..K
-  int levels;       // K
+  uint32_t blocks;  // 2x2x2 record blocks of levels 1..levels
+  int levels;       // K, or with FP32 records the last level
+  int half_levels;  // K: levels 1..K have FP16 records, K + 1..levels FP32 ones
   int log2n;
 };
 
@@ -505,7 +507,7 @@ __device__ __forceinline__ uint32_t half_bits(__half v) { return (uint32_t)__hal
 
 template <typename T>
 __global__ void __launch_bounds__(256) records_kernel(const T* __restrict__ mips, MipOffsets mo, RecordLevels rl,
-                                                      uint4* __restrict__ out) {
+                                                      uint4* __restrict__ out, uint4* __restrict__ wide) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= rl.blocks) return;
   // Level of block g: level l has max(n / 2, 1)^3 blocks and n^3 records
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(256) records_kernel(const T* __restrict__ mips
     const uint32_t nblocks = 1u << (3 * max(ln - 1, 0));
     if (level == rl.levels || g < bstart + nblocks) break;
     bstart += nblocks;
-    rstart += 1u << (3 * ln);
+    rstart = level == rl.half_levels ? 0u : rstart + (1u << (3 * ln));  // the FP32 records start over
     ++level;
     --ln;
   }
@@ -526,6 +528,23 @@ __global__ void __launch_bounds__(256) records_kernel(const T* __restrict__ mips
   const int x0 = (int)(block & (nb - 1)) << 1, y0 = (int)((block >> lb) & (nb - 1)) << 1,
             z0 = (int)(block >> (2 * lb)) << 1;
   const T* src = mips + pick(mo.off, level);
+  if constexpr (sizeof(T) == 4) {
+    if (level > rl.half_levels) {
+      for (int r = 0; r < 8; ++r) {
+        const int rx = x0 + (r & 1), ry = y0 + ((r >> 1) & 1), rz = z0 + (r >> 2);
+        if (rx >= n || ry >= n || rz >= n) continue;
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          w[j] = __float_as_uint(src[((size_t)min(rz + (j >> 2), n - 1) * n + min(ry + ((j >> 1) & 1), n - 1)) * n +
+                                     min(rx + (j & 1), n - 1)]);
+        uint4* to = wide + 2 * ((size_t)rstart + ((size_t)rz * n + ry) * n + rx);
+        to[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        to[1] = make_uint4(w[4], w[5], w[6], w[7]);
+      }
+      return;
+    }
+  }
   uint32_t h[3][3][3];
 #pragma unroll
   for (int dz = 0; dz < 3; ++dz)
@@ -554,24 +573,26 @@ __global__ void __launch_bounds__(256) records_kernel(const T* __restrict__ mips
 }  // namespace
 
 cudaError_t launch_build_records(cudaStream_t s, int n, const void* mips, const size_t* mip_offsets, int precision,
-                                 uint4* records, const uint32_t* record_offsets, int record_levels) {
+                                 uint4* records, const uint32_t* record_offsets, int record_levels, void* wide,
+                                 int n_levels) {
   if (record_levels <= 0) return cudaSuccess;
   MipOffsets mo{};
   RecordLevels rl{};
   for (int i = 0; i < kMaxVoxelLevels; ++i) mo.off[i] = mip_offsets[i];
-  rl.levels = record_levels;
+  rl.half_levels = record_levels;
+  rl.levels = wide ? n_levels - 1 : record_levels;
   while ((1 << (rl.log2n + 1)) <= n) ++rl.log2n;
   // the records of level l at record_offsets[l] = sum of (n >> j)^3 over j < l
-  for (int l = 1, ln = rl.log2n - 1; l <= record_levels; ++l, --ln) {
-    if (record_offsets[l] != (l == 1 ? 0u : record_offsets[l - 1] + (1u << (3 * (ln + 1)))))
+  for (int l = 1, ln = rl.log2n - 1; l <= rl.levels; ++l, --ln) {
+    if (l <= record_levels && record_offsets[l] != (l == 1 ? 0u : record_offsets[l - 1] + (1u << (3 * (ln + 1)))))
       return cudaErrorInvalidValue;
     rl.blocks += 1u << (3 * (ln > 0 ? ln - 1 : 0));
   }
   const dim3 grid((rl.blocks + 255) / 256);
   if (precision == DRV_PRECISION_BF16)
-    records_kernel<__half><<<grid, 256, 0, s>>>((const __half*)mips, mo, rl, records);
+    records_kernel<__half><<<grid, 256, 0, s>>>((const __half*)mips, mo, rl, records, nullptr);
   else
-    records_kernel<float><<<grid, 256, 0, s>>>((const float*)mips, mo, rl, records);
+    records_kernel<float><<<grid, 256, 0, s>>>((const float*)mips, mo, rl, records, (uint4*)wide);
   return cudaGetLastError();
 }
 

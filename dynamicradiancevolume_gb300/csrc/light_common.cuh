@@ -54,6 +54,12 @@ inline VoxelView make_voxel_view(const DrvConfig& cfg, const VoxelInputs& in) {
   for (int i = 1; i <= v.record_levels && i < 16; ++i)
     v.rbase[i] = (unsigned long long)reinterpret_cast<uintptr_t>(in.records + in.record_offsets[i]) -
                  (unsigned long long)tap_index_bias(L - i) * sizeof(uint4);
+  v.wide_levels = in.wide_records ? L : v.record_levels;
+  unsigned long long wide = (unsigned long long)reinterpret_cast<uintptr_t>(in.wide_records);
+  for (int i = v.record_levels + 1; i <= v.wide_levels && i < 16; ++i) {
+    v.rbase[i] = wide - (unsigned long long)tap_index_bias(L - i) * 32ull;
+    wide += (unsigned long long)kWideRecordBytes << (3 * (L - i));
+  }
   return v;
 }
 

@@ -15,7 +15,8 @@
 // 16-byte load instead of eight. With BF16 precision the texels are FP16 anyway and every level has
 // records; with FP32 precision levels 1..3 have them: a level-l texel is
 // k / 8^l (a mean of means of binary voxels) and FP16 holds it exactly for
-// 8^l <= 512, so the sample is the same FP32 value bit for bit.
+// 8^l <= 512, so the sample is the same FP32 value bit for bit; the few texels
+// of the levels above have FP32 records (32 bytes, two loads).
 #pragma once
 
 #include <cuda_fp16.h>
@@ -58,6 +59,7 @@ struct VoxelView {
   unsigned long long cbase;      // corners minus the taps' bias, as an address
   unsigned long long rbase[16];  // level l's corner-packed mip records minus 16 x the bias
   int record_levels;             // levels 1..record_levels have records
+  int wide_levels;               // levels record_levels + 1..wide_levels have FP32 records (rbase: minus 32 x the bias)
 };
 
 // Voxel loads of the sampler, for the cone pass's memory roofline: every
@@ -186,6 +188,7 @@ __device__ __forceinline__ float corner_blend(const CornerCoeffs& c, float x, fl
 // Where a kernel's sampler takes its constants from: computed from the view,
 // or (the cone pass) from a table in shared memory. Both give the same bits.
 struct ViewTable {
+  static constexpr bool kPlain = true;  // some levels may have no records
   __device__ __forceinline__ LevelConst level(const VoxelView& v, int l) const { return level_const(v, l); }
   __device__ __forceinline__ float corners(uint32_t byte, float x, float y, float z) const {
     // Empty space and solid are common: no expansion of the bits.
@@ -194,7 +197,9 @@ struct ViewTable {
     return corner_blend(corner_coeffs(byte), x, y, z);
   }
 };
+template <bool PLAIN>
 struct SharedTable {
+  static constexpr bool kPlain = PLAIN;
   const float4* a;  // [256] each: 16-byte rows, so that any eight rows of a
   const float4* b;  // quarter-warp spread over all banks
   const LevelConst* levels;
@@ -209,14 +214,15 @@ struct SharedTableStorage {
   LevelConst levels[kTableLevels];
 };
 // Filled by every thread of the CTA; the caller synchronises.
-__device__ __forceinline__ SharedTable fill_table(SharedTableStorage& s, const VoxelView& v) {
+template <bool PLAIN>
+__device__ __forceinline__ SharedTable<PLAIN> fill_table(SharedTableStorage& s, const VoxelView& v) {
   for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) {
     const CornerCoeffs c = corner_coeffs(i);
     s.a[i] = c.a;
     s.b[i] = c.b;
   }
   for (int l = (int)threadIdx.x; l <= v.max_level; l += (int)blockDim.x) s.levels[l] = level_const(v, l);
-  return SharedTable{s.a, s.b, s.levels};
+  return SharedTable<PLAIN>{s.a, s.b, s.levels};
 }
 
 // Level 0 at V: the load, and what its blend needs.
@@ -296,10 +302,18 @@ __device__ __forceinline__ float level_any_at(const VoxelView& v, const T& table
                                               bool& zero, R& reads) {
   zero = false;
   const LevelConst c = table.level(v, level);
-  if (level > v.record_levels) return level_n_at(v, level, c, V, reads);
-  const RecordLoad l = record_load(c, V, reads);
-  zero = l.zero();
-  return zero ? 0.0f : l.blend();
+  if (level <= v.record_levels) {
+    const RecordLoad l = record_load(c, V, reads);
+    zero = l.zero();
+    return zero ? 0.0f : l.blend();
+  }
+  if (T::kPlain && level > v.wide_levels) return level_n_at(v, level, c, V, reads);
+  // An FP32 record: the same eight texels.
+  reads.on_texels(8);
+  const Taps t = taps(V, c);
+  const float4* r = reinterpret_cast<const float4*>(c.base + (unsigned long long)tap_index(t, c) * 32ull);
+  const float4 lo = __ldg(r), hi = __ldg(r + 1);
+  return trilerp(lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w, t.ax, t.ay, t.az);
 }
 
 // Trilinear sample of one mip level >= 1 at s (no lod blend).
