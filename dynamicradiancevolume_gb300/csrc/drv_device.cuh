@@ -258,6 +258,14 @@ __device__ __forceinline__ uint32_t pack_cell(int x, int y, int z, int c) {
 // Atomic OR of device error bits.
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t bits) { atomicOr(err, bits); }
 
+// cachePrepareLighting.comp: dispatch size of the lighting pass.
+__device__ __forceinline__ void write_dispatch_size(DrvCacheCounter* counter, uint32_t max_caches) {
+  const uint32_t lit = min((uint32_t)max(counter->total_light_cache_count, 0), max_caches);
+  counter->groups_x = (lit + DRV_LIGHTING_THREADS_PER_GROUP - 1) / DRV_LIGHTING_THREADS_PER_GROUP;
+  counter->groups_y = 1;
+  counter->groups_z = 1;
+}
+
 // Cull record of a VPL as the light stage stores it (normal n, position p,
 // flux positive or not): the plane {n, -n . p + eps (1 + |p|_inf)}, or -inf in
 // w when it has no flux (no cache can see it). A cache c passes when

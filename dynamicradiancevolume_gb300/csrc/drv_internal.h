@@ -186,9 +186,15 @@ struct Context {
   uint32_t* atlas = nullptr;
   size_t atlas_words = 0;
   DrvCacheCounter* counter = nullptr;
-  uint32_t* scratch_words = nullptr;  // [0] alloc ticket, [1] device error bits, [4] input-check bits, [5] mips ticket
-  uint32_t* mips_ticket() const { return scratch_words + 5; }
-  uint32_t* input_err() const { return scratch_words + 4; }
+  // One allocation: 8 words that no allocation clears ([6] mips ticket, [7]
+  // input-check bits), then what each allocation clears in one go: the counter
+  // (4 words), 4 scratch words ([0] alloc ticket, [1] device error bits) and the
+  // atlas.
+  uint32_t* frame_mem = nullptr;
+  uint32_t* scratch_words = nullptr;
+  uint32_t* mips_ticket() const { return frame_mem + 6; }
+  uint32_t* input_err() const { return frame_mem + 7; }
+  size_t frame_clear_bytes() const { return (8 + atlas_words) * sizeof(uint32_t); }  // from counter
   // Voxels.
   uint32_t* voxel_bits = nullptr;  // followed by the tile list of drv_voxelize_triangles: head (16 bytes), entries
   size_t voxel_words = 0;
@@ -296,16 +302,19 @@ cudaError_t launch_build_corners(cudaStream_t s, int n, const uint32_t* bits, ui
 cudaError_t launch_build_records(cudaStream_t s, int n, const void* mips, const size_t* mip_offsets, int precision,
                                  uint4* records, const uint32_t* record_offsets, int record_levels, void* wide,
                                  int n_levels);
+// dispatch_size: followed by the launch that writes the lighting pass's dispatch
+// size (in a frame the light stage's first kernel writes it).
 cudaError_t launch_allocate(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,
                             const float* depth, int w, int h, uint32_t* atlas, void* entries, uint32_t entry_stride,
-                            DrvCacheCounter* counter, uint32_t* ticket, uint32_t* err, const float* ndc = nullptr);
+                            DrvCacheCounter* counter, uint32_t* err, const float* ndc, bool dispatch_size);
 // err: the context's device error word; with it, a stage without indirect
 // shadow runs from VPLs staged in shared memory (whose copy's bounded wait
-// reports there).
+// reports there). dispatch: where the stage writes its dispatch size
+// (cachePrepareLighting.comp), or nullptr.
 cudaError_t launch_light_caches(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const LightLaunch& ll,
                                 const DrvCacheCounter* counter, void* entries, uint32_t entry_stride,
                                 const VoxelInputs& vox, const LightScratch& scratch, int num_sms,
-                                uint32_t* err = nullptr);
+                                uint32_t* err = nullptr, DrvCacheCounter* dispatch = nullptr);
 // The learned visibility surrogate of a light stage: packed weights
 // (nullptr: plain cones), feature set (kFeature*), confidence threshold, the
 // device error word its bounded waits report to, and the timeout test hook
@@ -329,6 +338,7 @@ struct SplitKnobs {
   int gather_threads = 512;
   int gather_wait_test = 0;  // test hook: the gather's VPL copies are withheld (its bounded wait runs out)
   bool count_voxel_reads = false;
+  bool counters_clear = false;  // the pair list's counters are zero already (drv_frame clears them off the critical path)
 };
 
 // Split light stage: cull -> (cones | surrogate MLP + cones of the
@@ -337,19 +347,21 @@ bool light_split_supported(const DrvConfig& cfg, const LightLaunch& ll);
 cudaError_t launch_light_split(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const LightLaunch& ll,
                                const DrvCacheCounter* counter, void* entries, uint32_t entry_stride,
                                const VoxelInputs& vox, const PairList& pairs, const SurrogateArgs& sur,
-                               uint32_t* err, const SplitKnobs& knobs, int num_sms, cudaEvent_t* events = nullptr,
-                               cudaEvent_t voxels_ready = nullptr);
+                               uint32_t* err, const SplitKnobs& knobs, int num_sms, cudaEvent_t* events,
+                               cudaEvent_t voxels_ready, DrvCacheCounter* dispatch);
 cudaError_t launch_bruteforce_rsm(cudaStream_t s, const DrvPerFrame& f, const DrvGBufferView& g,
                                   const float* rough_metal, const LightLaunch& ll, int bf16, float* out_rgb,
                                   const float* srgb);
 // spec: the envmap atlas when specular is on, else nullptr.
 // err: device error word (DRV_DEVERR_BOUNDS for an atlas slot past the count).
+// after_light: the launch right before this one in the stream is the light
+// stage's last kernel; its tail is overlapped (programmatic dependent launch).
 // tensor_core: BF16 entries evaluated a warp's cells at a time on the tensor
 // cores instead of per pixel on the FP32 pipes (DrvTuning.tensor_core_apply).
 cudaError_t launch_apply(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,
                          const DrvGBufferView& g, const uint32_t* atlas, const void* entries, uint32_t entry_stride,
                          const DrvCacheCounter* counter, float* out_rgb, const float* srgb,
-                         const SpecView* spec = nullptr, uint32_t* err = nullptr, bool tensor_core = false);
+                         const SpecView* spec, uint32_t* err, bool tensor_core, bool after_light);
 // Sets DRV_DEVERR_NUMERIC in *word when any of n values (float, or half when
 // half is nonzero) is NaN or infinite.
 cudaError_t launch_scan_finite(cudaStream_t s, const void* data, size_t n, int half, uint32_t* word);

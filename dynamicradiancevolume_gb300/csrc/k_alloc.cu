@@ -1,8 +1,8 @@
 // k_alloc.cu — Renderer::AllocateCaches (renderer.cpp:951-992):
 // cacheGather.comp (16x16 workgroups, shared-memory neighbour dedupe, corner
 // lock by compare-and-swap, compaction by an atomic counter) and
-// cachePrepareLighting.comp (indirect-dispatch arguments, a one-thread
-// launch after it).
+// cachePrepareLighting.comp (indirect-dispatch arguments: a one-thread
+// launch after it, or in a frame the light stage's first kernel).
 #include "drv_device.cuh"
 #include "drv_internal.h"
 
@@ -130,17 +130,14 @@ __global__ void __launch_bounds__(kTile* kTile, 8) allocate_kernel(AllocParams p
 
 // cachePrepareLighting.comp: dispatch size of the lighting pass.
 __global__ void prepare_lighting_kernel(DrvCacheCounter* counter, uint32_t max_caches) {
-  const uint32_t lit = min((uint32_t)max(counter->total_light_cache_count, 0), max_caches);
-  counter->groups_x = (lit + DRV_LIGHTING_THREADS_PER_GROUP - 1) / DRV_LIGHTING_THREADS_PER_GROUP;
-  counter->groups_y = 1;
-  counter->groups_z = 1;
+  write_dispatch_size(counter, max_caches);
 }
 
 }  // namespace
 
 cudaError_t launch_allocate(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,
                             const float* depth, int w, int h, uint32_t* atlas, void* entries, uint32_t entry_stride,
-                            DrvCacheCounter* counter, uint32_t* /*ticket: unused*/, uint32_t* err, const float* ndc) {
+                            DrvCacheCounter* counter, uint32_t* err, const float* ndc, bool dispatch_size) {
   AllocParams p;
   p.rc = make_cell_recip(vol);
   p.ndc_x = ndc;
@@ -162,7 +159,7 @@ cudaError_t launch_allocate(cudaStream_t s, const DrvConfig& cfg, const DrvVolum
   p.err = err;
   dim3 block(kTile, kTile), grid((w + kTile - 1) / kTile, (h + kTile - 1) / kTile);
   allocate_kernel<<<grid, block, 0, s>>>(p);
-  prepare_lighting_kernel<<<1, 1, 0, s>>>(counter, cfg.max_caches);
+  if (dispatch_size) prepare_lighting_kernel<<<1, 1, 0, s>>>(counter, cfg.max_caches);
   return cudaGetLastError();
 }
 

@@ -168,7 +168,7 @@ __device__ __forceinline__ f3 lighting(const ApplyParams& p, const float wp[3], 
     } else if (BF16) {
       // 27 BF16 values from byte 4 of the 64-byte entry, coefficient-major.
       const uint4* e = reinterpret_cast<const uint4*>(p.entries + (size_t)(addr - 1u) * p.stride_floats);
-      const uint4 a = __ldg(e), b = __ldg(e + 1), cc = __ldg(e + 2), d = __ldg(e + 3);
+      const uint4 a = e[0], b = e[1], cc = e[2], d = e[3];
       const uint32_t q[16] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, cc.x, cc.y, cc.z, cc.w, d.x, d.y, d.z, d.w};
       float sh[27];
 #pragma unroll
@@ -190,7 +190,7 @@ __device__ __forceinline__ f3 lighting(const ApplyParams& p, const float wp[3], 
       }
     } else {
       const float4* e = reinterpret_cast<const float4*>(p.entries + (size_t)(addr - 1u) * p.stride_floats);
-      const float4 q1 = __ldg(e + 1), q2 = __ldg(e + 2), q3 = __ldg(e + 3);
+      const float4 q1 = e[1], q2 = e[2], q3 = e[3];
       // q1 = {SH1neg1, SH00_r}, q2 = {SH10, SH00_g}, q3 = {SH1pos1, SH00_b}
       erg = mul2(make_float2(q1.w, q2.w), pair(f0));
       erg = fma2(make_float2(q1.x, q1.y), pair(f1y), erg);
@@ -198,7 +198,7 @@ __device__ __forceinline__ f3 lighting(const ApplyParams& p, const float wp[3], 
       erg = fma2(make_float2(q3.x, q3.y), pair(f1x), erg);
       eb = __fmaf_rn(q3.z, f1x, __fmaf_rn(q2.z, f1z, __fmaf_rn(q1.z, f1y, __fmul_rn(q3.w, f0))));
       if (SH2) {
-        const float4 q4 = __ldg(e + 4), q5 = __ldg(e + 5), q6 = __ldg(e + 6), q7 = __ldg(e + 7);
+        const float4 q4 = e[4], q5 = e[5], q6 = e[6], q7 = e[7];
         // q4 = {SH2neg2, SH20_r}, q5 = {SH2neg1, SH20_g}, q6 = {SH2pos1, SH20_b}, q7 = {SH2pos2, pad}
         erg = fma2(make_float2(q4.x, q4.y), pair(f4), erg);
         erg = fma2(make_float2(q5.x, q5.y), pair(f5), erg);
@@ -264,6 +264,8 @@ __global__ void __launch_bounds__(256, SPEC ? 3 : 5) apply_kernel(ApplyParams p)
   // cacheApply.frag:304-307 (discard). A NaN depth counts as no geometry
   // too (the reference's test passes it and shades NaN).
   if (!(d >= 0.00001f)) {
+    // Every thread waits, so that this grid never ends before the light stage.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!p.out_add) store_output(p, i, mkf3(0.0f, 0.0f, 0.0f));
     return;
   }
@@ -278,10 +280,13 @@ __global__ void __launch_bounds__(256, SPEC ? 3 : 5) apply_kernel(ApplyParams p)
   const float inv_pi = 1.0f / DRV_SHADER_PI;
   const f3 a = load_albedo(p.albedo, p.albedo_format, p.srgb, i);
   f3 alb = mkf3(a.x * inv_pi, a.y * inv_pi, a.z * inv_pi);
-  const uint32_t n_caches = min((uint32_t)max(p.counter->total_light_cache_count, 0), p.max_caches);
   float wp[3];
   reconstruct_world(p.frame, x, y, p.w, p.h, d, wp);
   const int c = select_cascade(p.vol, p.n_cascades, wp);
+  // Up to here only the G-buffer is read; in a frame this grid starts while the
+  // light stage's last kernel finishes.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const uint32_t n_caches = min((uint32_t)max(p.counter->total_light_cache_count, 0), p.max_caches);
   EnvLookup q{};
   f3 spec_col = mkf3(0.0f, 0.0f, 0.0f);
   if (SPEC) {
@@ -437,6 +442,7 @@ __global__ void __launch_bounds__(256, 3) apply_tc_kernel(ApplyParams p) {
     ldsm_x4(ah[m], (uint32_t)__cvta_generic_to_shared(s_f[warp][0] + row * kTcRow + col));
     ldsm_x4(al[m], (uint32_t)__cvta_generic_to_shared(s_f[warp][1] + row * kTcRow + col));
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t n_caches = min((uint32_t)max(p.counter->total_light_cache_count, 0), p.max_caches);
   const int g = lane >> 2, t = lane & 3;
   const int aw = p.n_cascades * p.res;
@@ -490,9 +496,9 @@ __global__ void __launch_bounds__(256, 3) apply_tc_kernel(ApplyParams p) {
         const int k0 = 2 * t, k1 = 2 * t + 1;
 #pragma unroll
         for (int ch = 0; ch < 3; ++ch) {
-          const uint32_t v0 = k0 < NK ? __ldg(sh + 3 * k0 + ch) : 0u, v1 = k1 < NK ? __ldg(sh + 3 * k1 + ch) : 0u;
+          const uint32_t v0 = k0 < NK ? sh[3 * k0 + ch] : 0u, v1 = k1 < NK ? sh[3 * k1 + ch] : 0u;
           b0[ch] = v0 | v1 << 16;
-          b1[ch] = (SH2 && t == 0) ? (uint32_t)__ldg(sh + 24 + ch) : 0u;
+          b1[ch] = (SH2 && t == 0) ? (uint32_t)sh[24 + ch] : 0u;
         }
       }
       // Accumulators: lane (g, t) holds pixels 16m + g (+ 8) at corners 2t, 2t + 1.
@@ -561,7 +567,7 @@ __global__ void __launch_bounds__(256, 3) apply_tc_kernel(ApplyParams p) {
 cudaError_t launch_apply(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,
                          const DrvGBufferView& g, const uint32_t* atlas, const void* entries, uint32_t entry_stride,
                          const DrvCacheCounter* counter, float* out_rgb, const float* srgb, const SpecView* spec,
-                         uint32_t* err, bool tensor_core) {
+                         uint32_t* err, bool tensor_core, bool after_light) {
   ApplyParams p{};
   p.err = err;
   p.rc = make_cell_recip(vol);
@@ -607,15 +613,21 @@ cudaError_t launch_apply(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeIn
             : apply_kernel<false, false, true><<<grid, block, 0, s>>>(p);
     return cudaGetLastError();
   }
-  if (p.bf16 && tensor_core)
-    p.sh2 ? apply_tc_kernel<true><<<grid, block, 0, s>>>(p) : apply_tc_kernel<false><<<grid, block, 0, s>>>(p);
-  else if (p.bf16)
-    p.sh2 ? apply_kernel<true, true, false><<<grid, block, 0, s>>>(p)
-          : apply_kernel<true, false, false><<<grid, block, 0, s>>>(p);
-  else
-    p.sh2 ? apply_kernel<false, true, false><<<grid, block, 0, s>>>(p)
-          : apply_kernel<false, false, false><<<grid, block, 0, s>>>(p);
-  return cudaGetLastError();
+  auto launch = [&](void (*kernel)(ApplyParams)) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = after_light ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, p);
+  };
+  if (p.bf16 && tensor_core) return launch(p.sh2 ? apply_tc_kernel<true> : apply_tc_kernel<false>);
+  if (p.bf16) return launch(p.sh2 ? apply_kernel<true, true, false> : apply_kernel<true, false, false>);
+  return launch(p.sh2 ? apply_kernel<false, true, false> : apply_kernel<false, false, false>);
 }
 
 }  // namespace drv

@@ -81,6 +81,7 @@ StageParams make_stage_params(const DrvConfig& cfg, const DrvVolumeInfo& vol, co
   p.ev[4] = (float)std::sqrt(15.0 / (16.0 * kPi));
   p.spec = cfg.specular_envmap_size > 0;
   p.err = nullptr;
+  p.dispatch = nullptr;
   return p;
 }
 
@@ -132,6 +133,7 @@ constexpr int kCullWarps = kCullThreads / 32;
 template <bool BF16>
 __global__ void __launch_bounds__(kCullThreads) cull_kernel(StageParams p, PairList L) {
   pdl_wait_and_release();
+  note_dispatch_size(p);
   extern __shared__ uint32_t s_dyn[];  // [W] ballot words, [W] exclusive prefix of their popcounts
   __shared__ uint32_t s_warp[kCullWarps];
   __shared__ uint32_t s_base, s_count;
@@ -253,6 +255,7 @@ __device__ __forceinline__ void plane_tests(const float4 r, const float (&cx)[K]
 template <bool BF16, bool UNIT, bool COPY, int K>
 __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StageParams p, PairList L, int total_vpls) {
   pdl_wait_and_release();
+  note_dispatch_size(p);
   extern __shared__ float4 s_rec[];
   __shared__ uint32_t s_base[K], s_count[K];
   __shared__ __align__(8) uint64_t s_bar;
@@ -860,6 +863,8 @@ __global__ void __launch_bounds__(kUnshadowedThreads, 1) unshadowed_kernel(Fused
   constexpr bool KAHAN = BF16;
   constexpr int NV = NK * 3;
   const int lane = threadIdx.x & 31;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the apply's first loads overlap this grid's tail
+  note_dispatch_size(p);
   stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, 0);
   const bool ok = !staged || stage_vpls_wait(p, &s_bar, kGatherWaitCycles);
   const uint32_t n_units = ok ? cache_count(p) * (uint32_t)fp.n_chunks : 0u;
@@ -902,6 +907,7 @@ __global__ void __launch_bounds__(kUnshadowedThreads, 1) unshadowed_kernel(Fused
 template <int NK, bool BF16>
 __global__ void __launch_bounds__(kThreads, 8) light_kernel(FusedParams fp) {
   const StageParams& p = fp.s;
+  note_dispatch_size(p);
   constexpr bool KAHAN = BF16;
   __shared__ float s_acc[NK * 3 * kThreads * (KAHAN ? 2 : 1)];
   __shared__ int s_queue[kWarps][64];
@@ -1063,7 +1069,8 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
     cudaError_t r = begin(k);
     return r == cudaSuccess ? end(k) : r;
   };
-  cudaError_t e = cudaMemsetAsync(L.counters, 0, kPairCounters * sizeof(uint32_t), s);
+  cudaError_t e = knobs.counters_clear ? cudaSuccess
+                                       : cudaMemsetAsync(L.counters, 0, kPairCounters * sizeof(uint32_t), s);
   if (e != cudaSuccess || (e = begin(DRV_LK_CULL)) != cudaSuccess) return e;
   int total_vpls = 0;
   for (int l = 0; l < p.ll.n_lights; ++l) total_vpls += p.ll.lights[l].n_vpls;
@@ -1148,9 +1155,11 @@ int light_chunks(int total_blocks, int max_chunks) {
 
 cudaError_t launch_light_caches(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const LightLaunch& ll,
                                 const DrvCacheCounter* counter, void* entries, uint32_t entry_stride,
-                                const VoxelInputs& vox, const LightScratch& scratch, int num_sms, uint32_t* err) {
+                                const VoxelInputs& vox, const LightScratch& scratch, int num_sms, uint32_t* err,
+                                DrvCacheCounter* dispatch) {
   FusedParams fp;
   fp.s = make_stage_params(cfg, vol, ll, counter, entries, entry_stride, vox);
+  fp.s.dispatch = dispatch;
   fp.n_chunks = light_chunks(fp.s.total_blocks, scratch.max_chunks);
   fp.chunk_blocks = (fp.s.total_blocks + fp.n_chunks - 1) / fp.n_chunks;
   fp.scratch = scratch.partials;
@@ -1182,9 +1191,10 @@ cudaError_t launch_light_split(cudaStream_t s, const DrvConfig& cfg, const DrvVo
                                const DrvCacheCounter* counter, void* entries, uint32_t entry_stride,
                                const VoxelInputs& vox, const PairList& pairs, const SurrogateArgs& sur,
                                uint32_t* err, const SplitKnobs& knobs, int num_sms, cudaEvent_t* events,
-                               cudaEvent_t voxels_ready) {
+                               cudaEvent_t voxels_ready, DrvCacheCounter* dispatch) {
   StageParams p = make_stage_params(cfg, vol, ll, counter, entries, entry_stride, vox);
   p.err = err;
+  p.dispatch = dispatch;
   const bool bf16 = cfg.precision == DRV_PRECISION_BF16;
   if (cfg.sh_order == 2)
     return bf16 ? split_variant<9, true>(s, p, pairs, sur, knobs, num_sms, events, voxels_ready)

@@ -34,6 +34,7 @@ struct StageParams {
   float ev[5];  // ShEvaFactor0, 1, 2n2_p1_n1, 20, 2p2 (renderer.cpp:302-306)
   int spec;     // INDIRECT_SPECULAR: VPLs with a flux sum below 0.001 are skipped
   uint32_t* err;  // device error word for bounded waits (nullptr: none)
+  DrvCacheCounter* dispatch;  // where the stage's first kernel writes the dispatch size (nullptr: nowhere)
 };
 
 // Host: the device view of a voxel pyramid of resolution cfg.voxel_res.
@@ -119,6 +120,11 @@ cudaError_t launch_after(void (*kernel)(KArgs...), int blocks, int threads, size
 
 __device__ __forceinline__ uint32_t cache_count(const StageParams& p) {
   return min((uint32_t)max(p.counter->total_light_cache_count, 0), p.max_caches);
+}
+
+// The stage's first kernel: the dispatch size, where the frame wants it.
+__device__ __forceinline__ void note_dispatch_size(const StageParams& p) {
+  if (p.dispatch && blockIdx.x == 0 && threadIdx.x == 0) write_dispatch_size(p.dispatch, p.max_caches);
 }
 
 // Shadow block b (global index) -> light.
