@@ -107,20 +107,9 @@ __device__ __forceinline__ float cascade_transition(const DrvVolumeInfo& v, int 
   return fminf(fmaxf(t, 0.0f), 1.0f);
 }
 
-// clamp(ivec3(v), 0, res - 1), ivec3 truncating toward zero.
+// clamp(ivec3(v), 0, res - 1), ivec3 truncating toward zero (NaN: 0).
 __device__ __forceinline__ int trunc_clamp(float v, int res) {
-  if (!(v > 0.0f)) return 0;
-  if (v >= (float)(res - 1)) return res - 1;
-  return __float2int_rz(v);
-}
-
-// GetCache1DCoord, cacheGather.comp:20-30.
-__device__ __forceinline__ int cache_1d_coord(const DrvVolumeInfo& v, int res, int c, const float p[3]) {
-  const DrvCascade& k = v.cascades[c];
-  int ix = trunc_clamp(__fdiv_rn(__fsub_rn(p[0], k.min[0]), k.world_voxel_size), res);
-  int iy = trunc_clamp(__fdiv_rn(__fsub_rn(p[1], k.min[1]), k.world_voxel_size), res);
-  int iz = trunc_clamp(__fdiv_rn(__fsub_rn(p[2], k.min[2]), k.world_voxel_size), res);
-  return ix + iy * res + iz * res * res + c * res * res * res;
+  return __float2int_rz(fminf(fmaxf(v, 0.0f), (float)(res - 1)));
 }
 
 // Exact reciprocals of the divisors of the cascade arithmetic: where a
@@ -167,14 +156,10 @@ __device__ __forceinline__ float cascade_transition(const DrvVolumeInfo& v, cons
   return fminf(fmaxf(t, 0.0f), 1.0f);
 }
 
-__device__ __forceinline__ int cache_1d_coord(const DrvVolumeInfo& v, const CellRecip& r, int res, int c,
-                                              const float p[3]) {
-  const DrvCascade& k = v.cascades[c];
-  const float inv = r.inv_cell[c];
-  int ix = trunc_clamp(div_exact(__fsub_rn(p[0], k.min[0]), k.world_voxel_size, inv), res);
-  int iy = trunc_clamp(div_exact(__fsub_rn(p[1], k.min[1]), k.world_voxel_size, inv), res);
-  int iz = trunc_clamp(div_exact(__fsub_rn(p[2], k.min[2]), k.world_voxel_size, inv), res);
-  return ix + iy * res + iz * res * res + c * res * res * res;
+// Key of a cache cell (the allocation's, and the BF16 cache entries'): cascade-local corner coordinates (0..256,
+// 9 bits each) + cascade.
+__device__ __forceinline__ uint32_t pack_cell(int x, int y, int z, int c) {
+  return (uint32_t)x | (uint32_t)y << 9 | (uint32_t)z << 18 | (uint32_t)c << 27;
 }
 
 // G-buffer diffuse of pixel i (drv_albedo_format): linear F32 RGB, or SRGB8
@@ -248,12 +233,6 @@ __device__ __forceinline__ int sh_offset(int k, int ch) {
 // BF16 <-> FP32 (round to nearest even) as raw 16-bit storage.
 __device__ __forceinline__ uint16_t to_bf16(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float from_bf16(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
-
-// Cell key of a BF16 cache entry: cascade-local corner coordinates (0..256,
-// 9 bits each) + cascade.
-__device__ __forceinline__ uint32_t pack_cell(int x, int y, int z, int c) {
-  return (uint32_t)x | (uint32_t)y << 9 | (uint32_t)z << 18 | (uint32_t)c << 27;
-}
 
 // Atomic OR of device error bits.
 __device__ __forceinline__ void raise_error(uint32_t* err, uint32_t bits) { atomicOr(err, bits); }
