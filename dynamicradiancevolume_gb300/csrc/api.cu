@@ -141,8 +141,8 @@ cudaError_t alloc_pairs(Context* c, uint64_t cap) {
     c->pair_mem = nullptr;
   }
   // Every array starts on a 16-byte boundary (the unit list is read and
-  // written as 8-byte vectors).
-  const size_t slots = drv::gather_partial_slots(cap, c->cfg.max_caches);
+  // written as 16-byte vectors).
+  const size_t slots = drv::gather_unit_slots(cap, c->cfg.max_caches);
   const size_t mc = c->cfg.max_caches;
   size_t bytes = 0;
   auto take = [&bytes](size_t n) {
@@ -152,8 +152,8 @@ cudaError_t alloc_pairs(Context* c, uint64_t cap) {
   };
   const size_t o_cache = take(cap * 4), o_block = take(cap * 4), o_shadow = take(cap * 4),
                o_order = take(cap * 4), o_info = take(mc * 8),
-               o_counters = take(drv::kPairCounters * 4), o_tickets = take(mc * 4),
-               o_partials = take(slots * drv::kGatherSlotFloats * 4), o_units = take(slots * sizeof(uint2)),
+               o_counters = take(drv::kPairCounters * 4), o_range = take(mc * 8),
+               o_partials = take(slots * drv::kGatherSlotFloats * 4), o_units = take(slots * sizeof(uint4)),
                o_cls = take(cap);
   cudaError_t e = cudaMalloc(&c->pair_mem, bytes);
   if (e != cudaSuccess) return e;
@@ -165,10 +165,9 @@ cudaError_t alloc_pairs(Context* c, uint64_t cap) {
   c->pairs.order = reinterpret_cast<uint32_t*>(m + o_order);
   c->pairs.info = reinterpret_cast<uint32_t*>(m + o_info);
   c->pairs.counters = reinterpret_cast<uint32_t*>(m + o_counters);
-  c->pairs.tickets = reinterpret_cast<uint32_t*>(m + o_tickets);
+  c->pairs.unit_range = reinterpret_cast<uint2*>(m + o_range);
   c->pairs.partials = reinterpret_cast<float*>(m + o_partials);
-  c->pairs.partial_tail = (uint32_t)(cap / drv::kGatherChunk + 1);
-  c->pairs.units = reinterpret_cast<uint2*>(m + o_units);
+  c->pairs.units = reinterpret_cast<uint4*>(m + o_units);
   c->pairs.cls = reinterpret_cast<uint8_t*>(m + o_cls);
   c->pairs.cap = (uint32_t)cap;
   return cudaSuccess;

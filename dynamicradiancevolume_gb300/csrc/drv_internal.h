@@ -120,19 +120,18 @@ struct LightScratch {
 // ([4] zero), [5] pairs the surrogate evaluated, [6] the cone pass's work cursor,
 // [8 + c] pairs of class c, [8 + kConeClasses + c] class c's scatter cursor,
 // [kGatherUnitsCounter] the gather units listed in units.
-// The gather takes a cache's run in units of kGatherChunk pairs (units[u] =
-// {cache, unit index}, listed by the cull), a warp per unit; a cache of
-// several units sums their partials (partials: a slot per
-// unit, full units at the index of the multiple of kGatherChunk they cover,
-// each cache's last unit at partial_tail + cache) in unit order, done by the
-// unit that finishes last (tickets: per cache, zeroed by the cull).
+// The gather takes a cache's run in equal units (units[u] = {cache, first pair,
+// end, 1 if it is the cache's only one}, listed by the classification, a cache's
+// units next to each other, unit_range[cache] = {first, number}), a warp per unit;
+// the sums of a cache of several units go to partials (a slot per unit), and
+// gather_finish_kernel adds them to the entry in unit order.
 constexpr uint32_t kNoPair = 0xFFFFFFFFu;
 constexpr uint32_t kPairOverflow = 0xFFFFFFFFu;
 constexpr int kMaxSplitBlocks = 65536;  // shadow blocks per frame the split stage handles
 constexpr int kConeClasses = 32;
 constexpr int kGatherUnitsCounter = 8 + 2 * kConeClasses;
 constexpr int kPairCounters = kGatherUnitsCounter + 8;
-constexpr uint32_t kGatherChunk = 512;  // pairs per gather unit (a multiple of 32)
+constexpr uint32_t kGatherMinUnit = 64;  // fewest pairs a unit is planned for (a multiple of 32)
 constexpr int kGatherSlotFloats = 27;   // partial sums per unit slot (NK * 3 <= 27)
 struct PairList {
   uint32_t* cache;
@@ -142,16 +141,14 @@ struct PairList {
   uint8_t* cls;
   uint32_t* info;
   uint32_t* counters;
-  uint32_t* tickets;    // [max_caches]
-  float* partials;      // [partial_tail + max_caches][kGatherSlotFloats]
-  uint2* units;         // [partial_tail + max_caches]
-  uint32_t partial_tail;
+  uint2* unit_range;     // [max_caches]
+  float* partials;       // [gather_unit_slots][kGatherSlotFloats]
+  uint4* units;          // [gather_unit_slots]
   uint32_t cap;
 };
-// Slots of the gather's partial sums (and bound on its units) a pair list of
-// `cap` pairs needs.
-inline size_t gather_partial_slots(uint64_t cap, uint32_t max_caches) {
-  return (size_t)(cap / kGatherChunk + 1) + max_caches;
+// Bound on the gather's units for a pair list of `cap` pairs.
+inline size_t gather_unit_slots(uint64_t cap, uint32_t max_caches) {
+  return (size_t)(cap / kGatherMinUnit + 1) + max_caches;
 }
 
 // Ray frame of a pinhole camera: direction = normalize(fwd + nx*right + ny*up).

@@ -15,21 +15,23 @@
 //     VPL arrays, where the records do not fit) tests every block against
 //     the cache and writes the cache's contributing blocks, in block order,
 //     to one contiguous run of a global pair list (one atomic per cache
-//     claims it), and lists the cache's gather units;
+//     claims it);
 //  2. classify_kernel + scatter_kernel order the pairs by cone class (the
 //     number of steps the cone marches and whether it reaches mip samples),
 //     and cone_kernel (a thread per pair, persistent grid) traces the cones
-//     in that order and stores each pair's shadowing: every warp holds 32
+//     in that order and stores each pair's shadowing (the classification also
+//     lists the gather's units): every warp holds 32
 //     pairs, no lane idles on a block that needs no cone, and a warp's lanes
 //     march cones of one length along one sampling path; with the learned
 //     surrogate, the MLP (k_light_surrogate.cu) fills in the shadowing first
 //     and only the pairs it is not confident about are traced;
-//  3. gather_kernel (a warp per unit of up to kGatherChunk pairs of one
+//  3. gather_kernel (a warp per unit of pairs of one
 //     cache; one wave takes every cache at once): each lane gathers a fixed
 //     subset of the unit's pairs with their shadowing into SH partial sums
 //     in registers, reduced in a fixed order — the result does not depend on
 //     scheduling — and read-modify-written into the entry once (`+=`, as the
-//     reference's per-light dispatches accumulate).
+//     reference's per-light dispatches accumulate), the sums of a cache of
+//     several units by gather_finish_kernel.
 //
 // light_kernel, the single-launch form (warp per (cache, chunk) unit, cones
 // traced from a per-warp queue, ticketed chunk reduction), serves the
@@ -114,18 +116,6 @@ __device__ __forceinline__ void gather_block(const StageParams& p, float* acc, f
 }
 
 // ------------------------------------------------------------ split stage
-// Lists the gather units of cache c's run: one per kGatherChunk listed
-// pairs, one for a cache the list could not hold; and zeroes the cache's
-// ticket, so that a gather that stopped early (a timed-out copy) leaves no
-// count behind for the next stage.
-__device__ __forceinline__ void note_gather_units(const PairList& L, uint32_t c, uint32_t total, bool over) {
-  L.tickets[c] = 0u;
-  const uint32_t n = over ? 1u : (total + kGatherChunk - 1) / kGatherChunk;
-  if (!n) return;
-  const uint32_t base = atomicAdd(L.counters + kGatherUnitsCounter, n);
-  for (uint32_t k = 0; k < n; ++k) L.units[base + k] = make_uint2(c, k);
-}
-
 constexpr int kCullThreads = 256;
 constexpr int kCullWarps = kCullThreads / 32;
 
@@ -183,7 +173,6 @@ __global__ void __launch_bounds__(kCullThreads) cull_kernel(StageParams p, PairL
       const bool over = (uint64_t)base + total > (uint64_t)L.cap;
       L.info[2 * c] = base;
       L.info[2 * c + 1] = over ? kPairOverflow : total;
-      note_gather_units(L, c, total, over);
       s_base = base;
       s_count = over ? kPairOverflow : total;
     }
@@ -381,8 +370,7 @@ __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StagePara
         const bool over = (uint64_t)base + total > (uint64_t)L.cap;
         L.info[2 * c] = base;
         L.info[2 * c + 1] = over ? kPairOverflow : total;
-        note_gather_units(L, c, total, over);
-        s_base[k] = base;
+          s_base[k] = base;
         s_count[k] = over ? kPairOverflow : total;
       }
     }
@@ -428,6 +416,41 @@ __device__ __forceinline__ int cone_class(float light_dist, float inv_voxel, con
 }
 
 constexpr int kClassThreads = 256;
+constexpr int kListBlocks = 16;
+constexpr int kGatherWarps = 16;  // a gather CTA's (its smaller instance takes the same units)
+
+// Lists the gather units of every cache's run (one unit, without pairs, for a
+// cache the list could not hold), by `blocks` blocks. A unit costs
+// the gather about one round of 32 pairs of one VPL beside its pairs (its start,
+// reduction and sums), and a warp's last unit leaves it idle for half of one on
+// average: with T rounds a warp and R rounds a unit the pass takes about
+// T (1 + 1 / R) (1 + R / 2T), least at R = sqrt(2 T). Same pairs, same units: the
+// sums do not depend on scheduling. (512 pairs a unit, whatever the frame: 47, 65,
+// 72, 16 and 363 us for the gathers of 3.9, 5.5, 1.2 (of four VPLs), 0.5 and 40 M
+// pairs, against 43, 67, 55, 11 and 354. As a cache at a time per thread of the
+// cull's, or spread over all blocks here, the listing delays the pairs by 4 to 50 us.)
+__device__ __forceinline__ void list_gather_units(const StageParams& p, const PairList& L, uint32_t total,
+                                                  uint32_t gather_warps, float vpls_per_pair, uint32_t block,
+                                                  uint32_t blocks) {
+  const float rounds = (float)total / (32.0f * (float)gather_warps);
+  const uint32_t unit = max(kGatherMinUnit, 32u * (uint32_t)ceilf(sqrtf(2.0f * rounds / vpls_per_pair)));
+  const uint32_t n_caches = cache_count(p);
+  for (uint32_t c = block * blockDim.x + threadIdx.x; c < n_caches; c += blocks * blockDim.x) {
+    const uint32_t base = L.info[2 * c], count = L.info[2 * c + 1];
+    const bool over = count == kPairOverflow;
+    const uint32_t n = over ? 1u : (count + unit - 1) / unit;
+    const uint32_t first = n ? atomicAdd(L.counters + kGatherUnitsCounter, n) : 0u;
+    L.unit_range[c] = make_uint2(first, n);
+    if (over) {
+      L.units[first] = make_uint4(c, 0u, kPairOverflow, 1u);
+      continue;
+    }
+    const uint32_t pairs = n ? ((count + n - 1) / n + 31u) & ~31u : 0u;
+    for (uint32_t k = 0; k < n; ++k)
+      L.units[first + k] =
+          make_uint4(c, base + min(count, k * pairs), base + min(count, (k + 1) * pairs), n == 1u);
+  }
+}
 
 // Thread per listed pair: its cone class; class totals in counters[8 + c].
 // MARKED: only the pairs the surrogate left unconfident (cls 0) get a class;
@@ -437,14 +460,21 @@ constexpr int kClassThreads = 256;
 // thread, their loads together, are slower (614 and 629 us for the frame against
 // 610: fewer warps).
 template <bool BF16, bool MARKED>
-__global__ void __launch_bounds__(kClassThreads) classify_kernel(StageParams p, PairList L) {
+__global__ void __launch_bounds__(kClassThreads, 8) classify_kernel(StageParams p, PairList L, uint32_t gather_warps,
+                                                                 float vpls_per_pair) {
   pdl_wait_and_release();
   __shared__ uint32_t s_hist[kConeClasses];
   if (threadIdx.x < kConeClasses) s_hist[threadIdx.x] = 0u;
   __syncthreads();
   const uint32_t n = min(L.counters[0], L.cap);
+  // The last blocks list the gather's units beside the others' pairs.
+  const uint32_t list_blocks = min((uint32_t)kListBlocks, gridDim.x - 1u), pair_blocks = gridDim.x - list_blocks;
+  if (blockIdx.x >= pair_blocks || !list_blocks)
+    list_gather_units(p, L, n, gather_warps, vpls_per_pair, list_blocks ? blockIdx.x - pair_blocks : blockIdx.x,
+                      list_blocks ? list_blocks : gridDim.x);
+  if (blockIdx.x >= pair_blocks) return;
   const float inv_voxel = 1.0f / p.voxel_size, max_steps = (float)p.max_steps;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += pair_blocks * blockDim.x) {
     const uint32_t b = L.block[i];
     uint8_t c = 0xFF;
     if (b != kNoPair && (!MARKED || L.cls[i] != 0xFF)) {
@@ -700,17 +730,33 @@ __device__ __forceinline__ bool stage_vpls_wait(const StageParams& p, uint64_t* 
   return false;
 }
 
-// Warp per gather unit: kGatherChunk pairs of one cache's run (lane j sums
-// the unit's pairs j, j + 32, ... in order), or the whole cache when the list
-// could not hold it (the warp tests every block and traces the live ones'
+// Where a unit begins: its cache's position and each lane's first pair.
+struct GatherStart {
+  float x, y, z, shadow;
+  uint32_t block;
+};
+template <bool BF16>
+__device__ __forceinline__ GatherStart gather_start(const StageParams& p, const PairList& L, const uint4 unit,
+                                                    int lane) {
+  GatherStart s;
+  cache_position<BF16>(p, unit.x, s.x, s.y, s.z);
+  const uint32_t i = unit.y + lane;
+  const bool listed = unit.z != kPairOverflow && i < unit.z;
+  s.block = listed ? __ldg(L.block + i) : 0u;
+  s.shadow = listed ? __ldg(L.shadow + i) : 0.0f;
+  return s;
+}
+
+// Warp per gather unit: some pairs of one cache's run (lane j
+// sums the unit's pairs j, j + 32, ... in order), or the whole cache when the
+// list could not hold it (the warp tests every block and traces the live ones'
 // cones; the k-th live block goes to lane k mod 32, the lane its listed pair
-// would have had). The cull lists the units, so one wave of warps takes
+// would have had). The units are listed beforehand, so one wave of warps takes
 // every cache at once and a long run is spread over several warps. A cache
-// of one unit adds
-// its sums to the entry directly (`+=`, as the reference's per-light
-// dispatches accumulate); a longer one writes each unit's sums to its slot
-// and the unit that finishes last adds them in unit order: the result does
-// not depend on scheduling. One CTA per SM: its VPL copy (a bulk
+// of one unit adds its sums to the entry directly (`+=`, as the reference's
+// per-light dispatches accumulate); a longer one's are added by
+// gather_finish_kernel in unit order: the result does not depend on
+// scheduling. One CTA per SM: its VPL copy (a bulk
 // asynchronous copy per light, issued before the wait on the previous
 // kernel, since the VPLs were written before the light stage began) is
 // shared by all its warps. THREADS only sets the warps per CTA.
@@ -732,24 +778,24 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
   if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kGatherTestWaitCycles : kGatherWaitCycles)) return;
   const uint32_t n_units = L.counters[kGatherUnitsCounter];
   const uint32_t warps = gridDim.x * (THREADS / 32);
-  for (uint32_t u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); u < n_units; u += warps) {
-    const uint2 unit = L.units[u];
-    const uint32_t c = unit.x, k = unit.y;
-    const uint32_t first = L.info[2 * c], count = L.info[2 * c + 1];
-    const bool over = count == kPairOverflow;
-    const uint32_t units = over ? 1u : (count + kGatherChunk - 1) / kGatherChunk;
-    float cx, cy, cz;
-    cache_position<BF16>(p, c, cx, cy, cz);
+  uint32_t u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
+  if (u >= n_units) return;
+  uint4 unit = L.units[u];
+  GatherStart start = gather_start<BF16>(p, L, unit, lane);
+  for (;;) {
+    // the next unit's record is loaded while this unit is summed
+    const uint32_t u_next = u + warps;
+    const uint4 unit_next = u_next < n_units ? L.units[u_next] : unit;
+    const uint32_t hi = unit.z;
+    const float cx = start.x, cy = start.y, cz = start.z;
     float acc[NV], comp[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] = comp[q] = 0.0f;
-    const uint32_t lo = first + k * kGatherChunk;
-    if (!over) {
+    if (hi != kPairOverflow) {
       // the next pair's block and shadowing are loaded while this pair is summed
-      const uint32_t hi = first + min(count, (k + 1) * kGatherChunk);
-      uint32_t i = lo + lane;
-      uint32_t b_next = i < hi ? __ldg(L.block + i) : 0u;
-      float s_next = i < hi ? __ldg(L.shadow + i) : 0.0f;
+      uint32_t i = unit.y + lane;
+      uint32_t b_next = start.block;
+      float s_next = start.shadow;
       for (; i < hi; i += 32) {
         const uint32_t b = b_next;
         const float shadowing = s_next;
@@ -775,34 +821,45 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
         before += (uint32_t)n;
       }
     }
+    // and its cache and first pairs while this unit's sums are reduced
+    start = gather_start<BF16>(p, L, unit_next, lane);
     // Warp reduction of the NV sums: lane q ends up with coefficient q.
     float v[32];
 #pragma unroll
     for (int q = 0; q < 32; ++q) v[q] = q < NV ? (KAHAN ? __fsub_rn(acc[q], comp[q]) : acc[q]) : 0.0f;
     const float mine = warp_transpose_reduce<NV <= 16 ? 16 : 32>(v, lane);
-    float* entry = p.entries + (size_t)c * p.stride_floats;
-    if (units == 1u) {
-      if (lane < NV) add_to_entry<BF16>(entry, lane, mine);
-      continue;
-    }
-    auto slot_of = [&](uint32_t j) -> size_t {
-      return j + 1 < units ? (first + j * kGatherChunk + kGatherChunk - 1) / kGatherChunk
-                           : (size_t)L.partial_tail + c;
-    };
-    if (lane < NV) L.partials[slot_of(k) * kGatherSlotFloats + lane] = mine;
-    __threadfence();
-    __syncwarp();
-    uint32_t ticket = 0;
-    if (lane == 0) ticket = atomicAdd(L.tickets + c, 1u);
-    ticket = __shfl_sync(0xffffffffu, ticket, 0);
-    if (ticket + 1u != units) continue;
-    __threadfence();
     if (lane < NV) {
-      float sum = 0.0f;
-      for (uint32_t j = 0; j < units; ++j)
-        sum += j == k ? mine : __ldcg(L.partials + slot_of(j) * kGatherSlotFloats + lane);
-      add_to_entry<BF16>(entry, lane, sum);
+      if (unit.w)
+        add_to_entry<BF16>(p.entries + (size_t)unit.x * p.stride_floats, lane, mine);
+      else
+        L.partials[(size_t)u * kGatherSlotFloats + lane] = mine;
     }
+    if (u_next >= n_units) break;
+    u = u_next;
+    unit = unit_next;
+  }
+}
+
+// Warp per cache of several gather units: their sums, in unit order, into the
+// entry. A kernel of its own (about 3 us), since to count a cache's finished units
+// in the gather takes a fence, an atomic and a wait for every unit: 58 us for the
+// 3.9 M pairs of a 1080p frame and 456 us for 40 M, against 43 and 354. Bound by
+// the latency of its loads. Nothing is added after a gather whose copies timed out.
+constexpr int kFinishThreads = 128;
+template <int NK, bool BF16>
+__global__ void __launch_bounds__(kFinishThreads) gather_finish_kernel(StageParams p, PairList L) {
+  pdl_wait_and_release();
+  const int lane = threadIdx.x & 31;
+  const uint32_t n = cache_count(p), warps = gridDim.x * (kFinishThreads / 32);
+  if (p.err && (*p.err & DRV_DEVERR_TIMEOUT)) return;
+  for (uint32_t c = blockIdx.x * (kFinishThreads / 32) + (threadIdx.x >> 5); c < n; c += warps) {
+    const uint2 range = L.unit_range[c];
+    if (range.y < 2u || lane >= NK * 3) continue;
+    const float* slot = L.partials + (size_t)range.x * kGatherSlotFloats + lane;
+    float sum = 0.0f;
+#pragma unroll 4
+    for (uint32_t j = 0; j < range.y; ++j) sum += slot[j * kGatherSlotFloats];
+    add_to_entry<BF16>(p.entries + (size_t)c * p.stride_floats, lane, sum);
   }
 }
 
@@ -1099,8 +1156,10 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
     if ((e = end(DRV_LK_MLP)) != cudaSuccess) return e;
   }
   if ((e = begin(DRV_LK_CLASSIFY)) != cudaSuccess) return e;
-  e = sur.weights ? launch_persistent_after(classify_kernel<BF16, true>, kClassThreads, 0, s, num_sms, p, L)
-                  : launch_persistent_after(classify_kernel<BF16, false>, kClassThreads, 0, s, num_sms, p, L);
+  const int gather_threads = knobs.gather_threads == 256 ? 256 : kGatherWarps * 32;
+  e = launch_persistent_after(sur.weights ? classify_kernel<BF16, true> : classify_kernel<BF16, false>, kClassThreads, 0,
+                              s, num_sms, p, L, (uint32_t)(num_sms * kGatherWarps),
+                              (float)total_vpls / (float)p.total_blocks);
   if (e != cudaSuccess || (e = end(DRV_LK_CLASSIFY)) != cudaSuccess) return e;
   if ((e = begin(DRV_LK_SCATTER)) != cudaSuccess) return e;
   if ((e = launch_persistent_after(scatter_kernel, kClassThreads, 0, s, num_sms, L)) != cudaSuccess) return e;
@@ -1117,12 +1176,15 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
   {
     const uint32_t staged = gather_staged_vpls(p.ll, BF16);
     const size_t smem = (size_t)staged * vpl_bytes<BF16>();
-    auto kernel = knobs.gather_threads == 256 ? gather_kernel<NK, BF16, 256> : gather_kernel<NK, BF16, 512>;
+    auto kernel = gather_threads == 256 ? gather_kernel<NK, BF16, 256>
+                                         : gather_kernel<NK, BF16, kGatherWarps * 32>;
     if ((e = set_max_smem(reinterpret_cast<const void*>(kernel), kGatherStageBytes)) != cudaSuccess) return e;
-    e = launch_grid(kernel, knobs.gather_threads == 256 ? 256 : 512, smem, s, num_sms, knobs.gather_ctas_per_sm,
+    e = launch_grid(kernel, gather_threads, smem, s, num_sms, knobs.gather_ctas_per_sm,
                     true, p, L, staged, knobs.gather_wait_test);
   }
   if (e != cudaSuccess) return e;
+  if ((e = launch_grid(gather_finish_kernel<NK, BF16>, kFinishThreads, 0, s, num_sms, 8, true, p, L)) != cudaSuccess)
+    return e;
   return end(DRV_LK_GATHER);
 }
 
