@@ -417,6 +417,7 @@ __device__ __forceinline__ int cone_class(float light_dist, float inv_voxel, con
 
 constexpr int kClassThreads = 256;
 constexpr int kListBlocks = 16;
+constexpr uint32_t kGatherUnitBF16 = 512;
 constexpr int kGatherWarps = 16;  // a gather CTA's (its smaller instance takes the same units)
 
 // Lists the gather units of every cache's run (one unit, without pairs, for a
@@ -424,16 +425,21 @@ constexpr int kGatherWarps = 16;  // a gather CTA's (its smaller instance takes 
 // the gather about one round of 32 pairs of one VPL beside its pairs (its start,
 // reduction and sums), and a warp's last unit leaves it idle for half of one on
 // average: with T rounds a warp and R rounds a unit the pass takes about
-// T (1 + 1 / R) (1 + R / 2T), least at R = sqrt(2 T). Same pairs, same units: the
-// sums do not depend on scheduling. (512 pairs a unit, whatever the frame: 47, 65,
-// 72, 16 and 363 us for the gathers of 3.9, 5.5, 1.2 (of four VPLs), 0.5 and 40 M
-// pairs, against 43, 67, 55, 11 and 354. As a cache at a time per thread of the
-// cull's, or spread over all blocks here, the listing delays the pairs by 4 to 50 us.)
+// T (1 + 1 / R) (1 + R / 2T), least at R = sqrt(2 T) (FP32 entries, 512 pairs in
+// every frame: 65, 72 and 16 us for 5.5, 1.2 (of four VPLs) and 0.5 M pairs, so:
+// 67, 55 and 11). BF16 entries take units of 512 pairs in every frame: a sum that
+// differs by an FP32 rounding can round to the next BF16 value, so there a
+// cache's sums shall not depend on the other caches (as above: 43 us for 3.9 M
+// pairs against 47, 354 for 40 M against 363). Same pairs, same units: the sums do
+// not depend on scheduling. By every block, or by a thread of the cull, the
+// listing delays the pairs by 4 us, and 50 with 20 thousand caches.
+template <bool BF16>
 __device__ __forceinline__ void list_gather_units(const StageParams& p, const PairList& L, uint32_t total,
                                                   uint32_t gather_warps, float vpls_per_pair, uint32_t block,
                                                   uint32_t blocks) {
   const float rounds = (float)total / (32.0f * (float)gather_warps);
-  const uint32_t unit = max(kGatherMinUnit, 32u * (uint32_t)ceilf(sqrtf(2.0f * rounds / vpls_per_pair)));
+  const uint32_t unit =
+      BF16 ? kGatherUnitBF16 : max(kGatherMinUnit, 32u * (uint32_t)ceilf(sqrtf(2.0f * rounds / vpls_per_pair)));
   const uint32_t n_caches = cache_count(p);
   for (uint32_t c = block * blockDim.x + threadIdx.x; c < n_caches; c += blocks * blockDim.x) {
     const uint32_t base = L.info[2 * c], count = L.info[2 * c + 1];
@@ -445,7 +451,7 @@ __device__ __forceinline__ void list_gather_units(const StageParams& p, const Pa
       L.units[first] = make_uint4(c, 0u, kPairOverflow, 1u);
       continue;
     }
-    const uint32_t pairs = n ? ((count + n - 1) / n + 31u) & ~31u : 0u;
+    const uint32_t pairs = BF16 ? unit : n ? ((count + n - 1) / n + 31u) & ~31u : 0u;
     for (uint32_t k = 0; k < n; ++k)
       L.units[first + k] =
           make_uint4(c, base + min(count, k * pairs), base + min(count, (k + 1) * pairs), n == 1u);
@@ -470,7 +476,7 @@ __global__ void __launch_bounds__(kClassThreads, 8) classify_kernel(StageParams 
   // The last blocks list the gather's units beside the others' pairs.
   const uint32_t list_blocks = min((uint32_t)kListBlocks, gridDim.x - 1u), pair_blocks = gridDim.x - list_blocks;
   if (blockIdx.x >= pair_blocks || !list_blocks)
-    list_gather_units(p, L, n, gather_warps, vpls_per_pair, list_blocks ? blockIdx.x - pair_blocks : blockIdx.x,
+    list_gather_units<BF16>(p, L, n, gather_warps, vpls_per_pair, list_blocks ? blockIdx.x - pair_blocks : blockIdx.x,
                       list_blocks ? list_blocks : gridDim.x);
   if (blockIdx.x >= pair_blocks) return;
   const float inv_voxel = 1.0f / p.voxel_size, max_steps = (float)p.max_steps;
@@ -843,7 +849,7 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
 // Warp per cache of several gather units: their sums, in unit order, into the
 // entry. A kernel of its own (about 3 us), since to count a cache's finished units
 // in the gather takes a fence, an atomic and a wait for every unit: 58 us for the
-// 3.9 M pairs of a 1080p frame and 456 us for 40 M, against 43 and 354. Bound by
+// 3.9 M pairs of a 1080p frame and 456 us for 40 M, against 47 and 363. Bound by
 // the latency of its loads. Nothing is added after a gather whose copies timed out.
 constexpr int kFinishThreads = 128;
 template <int NK, bool BF16>
