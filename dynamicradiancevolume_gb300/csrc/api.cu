@@ -534,9 +534,10 @@ drv_status drv_raster_rsm(DrvContext* ctx, const DrvMesh* mesh, const DrvSpotLig
                     "raster_rsm");
 }
 
-// ShadowMap::PrepareRSM (renderer.cpp:1300-1339): successive 2x2 reductions,
-// down to the deepest level the light reads (read lod + shadow lod).
-drv_status drv_prepare_rsm(DrvContext* ctx, int32_t li, const DrvSpotLight* L, const DrvRSMView* v) {
+namespace {
+
+// Checks light li's RSM view and notes its chain.
+drv_status note_rsm(DrvContext* ctx, int32_t li, const DrvSpotLight* L, const DrvRSMView* v) {
   if (!ctx || !L || !v || !v->flux || !v->normal || !v->depth_lin_sq) return DRV_ERR_INVALID_ARG;
   if (li < 0 || li >= ctx->cfg.max_lights) return fail(ctx, DRV_ERR_INVALID_ARG, "light index out of range");
   const int R = v->resolution;
@@ -565,43 +566,93 @@ drv_status drv_prepare_rsm(DrvContext* ctx, int32_t li, const DrvSpotLight* L, c
     DRV_TRY_CUDA(ctx, drv::launch_scan_finite(ctx->s(), v->flux, n * 3, ch.half0, ctx->input_err()));
     DRV_TRY_CUDA(ctx, drv::launch_scan_finite(ctx->s(), v->depth_lin_sq, n * 2, ch.half0, ctx->input_err()));
   }
-  // The chain in launches of up to three passes each (launch_rsm_chain).
-  for (int k = 0; k < deepest; k += 3) {
-    const int passes = deepest - k < 3 ? deepest - k : 3;
-    float* fo[3] = {};
-    int16_t* no[3] = {};
-    float* dlo[3] = {};
-    for (int q = 0; q < passes; ++q) {
-      fo[q] = static_cast<float*>(ch.flux[k + 1 + q]);
-      no[q] = ch.normal[k + 1 + q];
-      dlo[q] = static_cast<float*>(ch.dls[k + 1 + q]);
+  return DRV_OK;
+}
+
+// The chains of lights first .. first + n - 1, as noted: in launches of up to
+// three passes each (launch_rsm_chain), the lights with as many passes left
+// together.
+drv_status reduce_rsms(DrvContext* ctx, int first, int n) {
+  for (int k = 0;; k += 3) {
+    bool any = false;
+    for (int passes = 1; passes <= 3; ++passes) {
+      drv::RsmChainArgs lights[DRV_MAX_LIGHTS] = {};
+      int count = 0;
+      for (int li = first; li < first + n; ++li) {
+        const drv::RsmChain& ch = ctx->rsm[li];
+        if (std::min(3, ch.n_levels - 1 - k) != passes) continue;
+        drv::RsmChainArgs& a = lights[count++];
+        a.res = ch.res0 >> k;
+        a.flux = ch.flux[k];
+        a.nrm = ch.normal[k];
+        a.dls = ch.dls[k];
+        a.src_half = ch.half(k);
+        for (int q = 0; q < passes; ++q) {
+          a.fo[q] = static_cast<float*>(ch.flux[k + 1 + q]);
+          a.no[q] = ch.normal[k + 1 + q];
+          a.dlo[q] = static_cast<float*>(ch.dls[k + 1 + q]);
+        }
+      }
+      if (!count) continue;
+      any = true;
+      DRV_TRY_CUDA(ctx, drv::launch_rsm_chain(ctx->s(), lights, count, passes));
     }
-    DRV_TRY_CUDA(ctx, drv::launch_rsm_chain(ctx->s(), R >> k, passes, ch.flux[k], ch.normal[k], ch.dls[k], ch.half(k),
-                                            fo, no, dlo));
+    if (!any) return DRV_OK;
+  }
+}
+
+// The VPLs of lights first .. first + n - 1 (L: the first one's) from their chains.
+drv_status extract_vpls(DrvContext* ctx, int first, int n, const DrvSpotLight* lights) {
+  drv::ExtractArgs args[DRV_MAX_LIGHTS] = {};
+  for (int q = 0; q < n; ++q) {
+    const int li = first + q;
+    const DrvSpotLight& L = lights[q];
+    const drv::RsmChain& ch = ctx->rsm[li];
+    if (ch.res0 != L.rsm_render_resolution || ch.n_levels < 1)
+      return fail(ctx, DRV_ERR_INVALID_ARG, "drv_prepare_rsm must run for this light first");
+    const int R = L.rsm_read_resolution;
+    const int read_lod = ilog2(ch.res0 / R);
+    const int shadow_level = read_lod + (int)L.indirect_shadow_lod;
+    if (shadow_level >= ch.n_levels) return fail(ctx, DRV_ERR_INVALID_ARG, "RSM chain too short for the shadow lod");
+    if (L.indirect_shadow_sample_interval < 1) return DRV_ERR_INVALID_ARG;
+    drv::ExtractArgs& a = args[q];
+    a.L = L;
+    a.R = R;
+    a.flux = ch.flux[read_lod];
+    a.nrm = ch.normal[read_lod];
+    a.dls = ch.dls[read_lod];
+    a.read_half = ch.half(read_lod);
+    a.dls_shadow = ch.dls[shadow_level];
+    a.shadow_half = ch.half(shadow_level);
+    a.vpls = ctx->vpls[li];
+    a.cones = ctx->cones[li];
+    a.records = ctx->vpl_records[li];
+    a.steps = ctx->cone_steps[li];
+  }
+  DRV_TRY_CUDA(ctx, drv::launch_extract_vpls(ctx->s(), args, n, ctx->cfg.precision));
+  for (int q = 0; q < n; ++q) {
+    const int li = first + q, R = lights[q].rsm_read_resolution, interval = lights[q].indirect_shadow_sample_interval;
+    ctx->n_vpls[li] = R * R;
+    ctx->interval[li] = interval;
+    ctx->n_cones[li] = (R * R + interval - 1) / interval;
+    if (li + 1 > ctx->n_lights) ctx->n_lights = li + 1;
   }
   return DRV_OK;
+}
+
+}  // namespace
+
+// ShadowMap::PrepareRSM (renderer.cpp:1300-1339): successive 2x2 reductions,
+// down to the deepest level the light reads (read lod + shadow lod).
+drv_status drv_prepare_rsm(DrvContext* ctx, int32_t li, const DrvSpotLight* L, const DrvRSMView* v) {
+  const drv_status st = note_rsm(ctx, li, L, v);
+  return st == DRV_OK ? reduce_rsms(ctx, li, 1) : st;
 }
 
 drv_status drv_extract_vpls(DrvContext* ctx, int32_t li, const DrvSpotLight* L) {
   if (!ctx || !L) return DRV_ERR_INVALID_ARG;
   if (li < 0 || li >= ctx->cfg.max_lights) return fail(ctx, DRV_ERR_INVALID_ARG, "light index out of range");
-  drv::RsmChain& ch = ctx->rsm[li];
-  if (ch.res0 != L->rsm_render_resolution || ch.n_levels < 1)
-    return fail(ctx, DRV_ERR_INVALID_ARG, "drv_prepare_rsm must run for this light first");
-  const int R = L->rsm_read_resolution;
-  const int read_lod = ilog2(ch.res0 / R);
-  const int shadow_level = read_lod + (int)L->indirect_shadow_lod;
-  if (shadow_level >= ch.n_levels) return fail(ctx, DRV_ERR_INVALID_ARG, "RSM chain too short for the shadow lod");
-  if (L->indirect_shadow_sample_interval < 1) return DRV_ERR_INVALID_ARG;
-  DRV_TRY_CUDA(ctx, drv::launch_extract_vpls(ctx->s(), *L, R, ch.flux[read_lod], ch.normal[read_lod], ch.dls[read_lod],
-                                             ch.half(read_lod), ch.dls[shadow_level], ch.half(shadow_level),
-                                             ctx->vpls[li], ctx->cones[li], ctx->cfg.precision,
-                                             ctx->vpl_records[li], ctx->cone_steps[li]));
-  ctx->n_vpls[li] = R * R;
-  ctx->interval[li] = L->indirect_shadow_sample_interval;
-  ctx->n_cones[li] = (R * R + L->indirect_shadow_sample_interval - 1) / L->indirect_shadow_sample_interval;
-  if (li + 1 > ctx->n_lights) ctx->n_lights = li + 1;
-  return DRV_OK;
+  return extract_vpls(ctx, li, 1, L);
 }
 
 drv_status drv_voxelize(DrvContext* ctx, const DrvScene* scene, const DrvVolumeInfo* vol) {
@@ -889,10 +940,9 @@ drv_status drv_frame(DrvContext* ctx, const DrvScene* scene, const DrvGBufferVie
   if (ctx->cfg.indirect_shadow && ctx->tuning.light_path != DRV_LIGHT_PATH_SINGLE)
     st = cuda_check(ctx, cudaMemsetAsync(ctx->pairs.counters, 0, drv::kPairCounters * sizeof(uint32_t), ctx->s()),
                     "clear the pair counters");
-  for (int l = 0; l < n_lights && st == DRV_OK; ++l) {
-    st = drv_prepare_rsm(ctx, l, &lights[l], &rsms[l]);
-    if (st == DRV_OK) st = drv_extract_vpls(ctx, l, &lights[l]);
-  }
+  for (int l = 0; l < n_lights && st == DRV_OK; ++l) st = note_rsm(ctx, l, &lights[l], &rsms[l]);
+  if (st == DRV_OK) st = reduce_rsms(ctx, 0, n_lights);
+  if (st == DRV_OK && n_lights > 0) st = extract_vpls(ctx, 0, n_lights, lights);
   ctx->cur = ctx->side[1];
   if (st == DRV_OK && ctx->cfg.indirect_shadow) {
     st = drv_voxelize(ctx, scene, vol);

@@ -279,11 +279,33 @@ cudaError_t launch_raster_rsm(cudaStream_t s, const DrvMesh& mesh, const DrvSpot
                               uint4* big, DrvRSMOut out, int num_sms);
 // Up to three RSM downsample passes res -> res/2 -> ... in one launch;
 // fo/no/dlo[k] receive level k + 1 (F32 flux and (d, d^2), RG16I normals).
-cudaError_t launch_rsm_chain(cudaStream_t s, int res, int passes, const void* flux, const int16_t* nrm,
-                             const void* dls, int src_half, float* const* fo, int16_t* const* no, float* const* dlo);
-cudaError_t launch_extract_vpls(cudaStream_t s, const DrvSpotLight& L, int res, const void* flux, const int16_t* nrm,
-                                const void* dls, int read_half, const void* dls_shadow, int shadow_half, void* vpls,
-                                DrvShadowCone* cones, int precision, float4* records, float4* steps);
+// One light's share of an RSM chain launch, and of an extraction.
+struct RsmChainArgs {
+  int res;  // source resolution
+  const void* flux;
+  const int16_t* nrm;
+  const void* dls;
+  int src_half;
+  float* fo[3];
+  int16_t* no[3];
+  float* dlo[3];
+};
+struct ExtractArgs {
+  DrvSpotLight L;
+  int R;
+  const void* flux;
+  const int16_t* nrm;
+  const void* dls;
+  int read_half;
+  const void* dls_shadow;
+  int shadow_half;
+  void* vpls;
+  DrvShadowCone* cones;
+  float4* records;
+  float4* steps;
+};
+cudaError_t launch_rsm_chain(cudaStream_t s, const RsmChainArgs* lights, int n_lights, int passes);
+cudaError_t launch_extract_vpls(cudaStream_t s, const ExtractArgs* lights, int n_lights, int precision);
 cudaError_t launch_voxelize(cudaStream_t s, const DrvBox* boxes, int n_boxes, const DrvVolumeInfo& vol, int n,
                             uint32_t* bits);
 cudaError_t launch_voxelize_triangles(cudaStream_t s, const float* positions, int n_vertices, const uint32_t* indices,

@@ -50,3 +50,34 @@ def test_frame_matches_its_stages(lights, shadow, per_light, single, lib, cuda):
         assert not p.out.any()
         p.depth.copy_(depth)
     p.close()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+def test_lights_of_different_resolutions_share_launches(bf16, lib, cuda):
+    """A frame's RSM chains and extractions run all lights per launch, those with
+    as many passes left together: the VPLs and shadow cones of lights that read
+    different levels of their chains are bit for bit those of the calls per light."""
+    w = pipeline.scaled(pipeline.WORKLOADS["c1_small"], width=64, height=64, n_lights=4, rsm_resolution=64,
+                        rsm_read_lod=0, precision=abi.PRECISION_BF16 if bf16 else abi.PRECISION_FP32)
+    p = pipeline.Pipeline(pipeline.host_frame(w, seed=2))
+    p.raycast_inputs()
+    for l, (read, shadow_lod) in enumerate([(64, 0), (4, 1), (16, 1), (8, 0)]):  # 0, 5, 3 and 3 passes
+        p.hf.lights[l].rsm_read_resolution = read
+        p.hf.lights[l].indirect_shadow_lod = shadow_lod
+        p.hf.lights[l].indirect_shadow_sample_interval = 4 ** shadow_lod
+    p.prepare_and_extract()
+    p.sync()
+
+    def state():
+        b = p.buffers()
+        return [(p._dev_tensor(b.vpls[l], b.n_vpls[l] * (8 if bf16 else 12), p.torch.int32).cpu().numpy(),
+                 p._dev_tensor(b.cones[l], b.n_vpls[l] // 4 ** shadow * 4, p.torch.int32).cpu().numpy())
+                for l, shadow in enumerate((0, 1, 1, 0))]
+
+    ref = state()
+    p.frame()
+    p.sync()
+    got = state()
+    for (v0, c0), (v1, c1) in zip(ref, got):
+        assert np.any(v0) and np.array_equal(v0, v1) and np.array_equal(c0, c1)
+    p.close()
