@@ -441,11 +441,24 @@ __device__ __forceinline__ void list_gather_units(const StageParams& p, const Pa
   const uint32_t unit =
       BF16 ? kGatherUnitBF16 : max(kGatherMinUnit, 32u * (uint32_t)ceilf(sqrtf(2.0f * rounds / vpls_per_pair)));
   const uint32_t n_caches = cache_count(p);
-  for (uint32_t c = block * blockDim.x + threadIdx.x; c < n_caches; c += blocks * blockDim.x) {
-    const uint32_t base = L.info[2 * c], count = L.info[2 * c + 1];
+  const int lane = threadIdx.x & 31;
+  for (uint32_t c0 = block * blockDim.x + (threadIdx.x & ~31u); c0 < n_caches; c0 += blocks * blockDim.x) {
+    const uint32_t c = c0 + lane;
+    const uint2 info = c < n_caches ? *reinterpret_cast<const uint2*>(L.info + 2 * c) : make_uint2(0u, 0u);
+    const uint32_t base = info.x, count = info.y;
     const bool over = count == kPairOverflow;
     const uint32_t n = over ? 1u : (count + unit - 1) / unit;
-    const uint32_t first = n ? atomicAdd(L.counters + kGatherUnitsCounter, n) : 0u;
+    // one count per warp: the lanes' units follow each other
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    uint32_t first = 0;
+    if (lane == 31 && incl) first = atomicAdd(L.counters + kGatherUnitsCounter, incl);
+    first = __shfl_sync(0xffffffffu, first, 31) + incl - n;
+    if (c >= n_caches) continue;
     L.unit_range[c] = make_uint2(first, n);
     if (over) {
       L.units[first] = make_uint4(c, 0u, kPairOverflow, 1u);
@@ -462,7 +475,8 @@ __device__ __forceinline__ void list_gather_units(const StageParams& p, const Pa
 // MARKED: only the pairs the surrogate left unconfident (cls 0) get a class;
 // the others keep 0xFF and are neither ordered nor traced. Bound by the
 // latency of its dependent loads; 3.9 M pairs: 37 -> 24 us (230 instructions a
-// pair with the cone's step rule evaluated in full). Two or four pairs per
+// pair with the cone's step rule evaluated in full); 40 M: 206 -> 186 us with the
+// next pair's block and cache loaded ahead. Two or four pairs per
 // thread, their loads together, are slower (614 and 629 us for the frame against
 // 610: fewer warps).
 template <bool BF16, bool MARKED>
@@ -480,12 +494,20 @@ __global__ void __launch_bounds__(kClassThreads, 8) classify_kernel(StageParams 
                       list_blocks ? list_blocks : gridDim.x);
   if (blockIdx.x >= pair_blocks) return;
   const float inv_voxel = 1.0f / p.voxel_size, max_steps = (float)p.max_steps;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += pair_blocks * blockDim.x) {
-    const uint32_t b = L.block[i];
+  // the next pair's block and cache are loaded while this pair is classified
+  const uint32_t stride = pair_blocks * blockDim.x;
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t b_next = i < n ? L.block[i] : kNoPair, cache_next = i < n ? L.cache[i] : 0u;
+  for (; i < n; i += stride) {
+    const uint32_t b = b_next, cache = cache_next;
+    if (i + stride < n) {
+      b_next = L.block[i + stride];
+      cache_next = L.cache[i + stride];
+    }
     uint8_t c = 0xFF;
     if (b != kNoPair && (!MARKED || L.cls[i] != 0xFF)) {
       float cx, cy, cz;
-      cache_position<BF16>(p, L.cache[i], cx, cy, cz);
+      cache_position<BF16>(p, cache, cx, cy, cz);
       const int l = block_light(p, (int)b), lb = (int)b - p.block_base[l];
       const float4 cone = __ldg(reinterpret_cast<const float4*>(p.ll.lights[l].cones) + lb);
       const float4 st = __ldg(p.ll.lights[l].steps + lb);
