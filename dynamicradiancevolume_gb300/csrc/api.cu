@@ -885,7 +885,7 @@ drv_status apply(DrvContext* ctx, const DrvGBufferView* g, const DrvPerFrame* f,
                                            ctx->entry_stride, ctx->counter, out_rgb, ctx->srgb,
                                            ctx->spec_env ? &sv : nullptr, ctx->scratch_words + 1,
                                            ctx->tuning.tensor_core_apply != 0,
-                                           after_light && !ctx->spec_env && !ctx->tuning.check_inputs),
+                                           after_light && !ctx->tuning.check_inputs),
                     "apply");
 }
 

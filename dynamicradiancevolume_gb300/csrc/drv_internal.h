@@ -374,7 +374,8 @@ cudaError_t launch_bruteforce_rsm(cudaStream_t s, const DrvPerFrame& f, const Dr
 // spec: the envmap atlas when specular is on, else nullptr.
 // err: device error word (DRV_DEVERR_BOUNDS for an atlas slot past the count).
 // after_light: the launch right before this one in the stream is the light
-// stage's last kernel; its tail is overlapped (programmatic dependent launch).
+// stage's last kernel or the envmaps' preparation; its tail is overlapped
+// (programmatic dependent launch).
 // tensor_core: BF16 entries evaluated a warp's cells at a time on the tensor
 // cores instead of per pixel on the FP32 pipes (DrvTuning.tensor_core_apply).
 cudaError_t launch_apply(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeInfo& vol, const DrvPerFrame& f,

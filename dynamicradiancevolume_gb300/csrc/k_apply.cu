@@ -93,7 +93,7 @@ __device__ __forceinline__ f3 env_bilinear(const uint2* half, const EnvTaps& t) 
   f3 r = mkf3(0.0f, 0.0f, 0.0f);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const uint2 q = __ldg(half + t.at[k]);
+    const uint2 q = half[t.at[k]];
     const float2 rg = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
     const float b = __low2float(*reinterpret_cast<const __half2*>(&q.y));
     r = mkf3(r.x + t.w[k] * rg.x, r.y + t.w[k] * rg.y, r.z + t.w[k] * b);
@@ -601,18 +601,6 @@ cudaError_t launch_apply(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeIn
   p.out_half = cfg.output_format == DRV_OUTPUT_RGBA16F;
   p.out_add = cfg.output_blend == DRV_OUTPUT_ADD;
   dim3 block(16, 16), grid((g.width + 15) / 16, (g.height + 15) / 16);
-  if (spec) {
-    p.spec = *spec;
-    p.rough_metal = g.rough_metal;
-    p.rm_f32 = g.rough_metal_format == DRV_ROUGH_METAL_F32;
-    if (p.bf16)
-      p.sh2 ? apply_kernel<true, true, true><<<grid, block, 0, s>>>(p)
-            : apply_kernel<true, false, true><<<grid, block, 0, s>>>(p);
-    else
-      p.sh2 ? apply_kernel<false, true, true><<<grid, block, 0, s>>>(p)
-            : apply_kernel<false, false, true><<<grid, block, 0, s>>>(p);
-    return cudaGetLastError();
-  }
   auto launch = [&](void (*kernel)(ApplyParams)) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -625,6 +613,13 @@ cudaError_t launch_apply(cudaStream_t s, const DrvConfig& cfg, const DrvVolumeIn
     cfg.numAttrs = after_light ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, p);
   };
+  if (spec) {
+    p.spec = *spec;
+    p.rough_metal = g.rough_metal;
+    p.rm_f32 = g.rough_metal_format == DRV_ROUGH_METAL_F32;
+    if (p.bf16) return launch(p.sh2 ? apply_kernel<true, true, true> : apply_kernel<true, false, true>);
+    return launch(p.sh2 ? apply_kernel<false, true, true> : apply_kernel<false, false, true>);
+  }
   if (p.bf16 && tensor_core) return launch(p.sh2 ? apply_tc_kernel<true> : apply_tc_kernel<false>);
   if (p.bf16) return launch(p.sh2 ? apply_kernel<true, true, false> : apply_kernel<true, false, false>);
   return launch(p.sh2 ? apply_kernel<false, true, false> : apply_kernel<false, false, false>);
