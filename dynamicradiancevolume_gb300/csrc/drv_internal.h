@@ -356,6 +356,7 @@ struct SplitKnobs {
   int cull_caches_per_pass = 4;
   int gather_threads = 512;
   int gather_wait_test = 0;  // test hook: the gather's VPL copies are withheld (its bounded wait runs out)
+  int cull_wait_test = 0;    // test hook: the cull's record copies are withheld
   bool count_voxel_reads = false;
   bool counters_clear = false;  // the pair list's counters are zero already (drv_frame clears them off the critical path)
 };

@@ -241,8 +241,30 @@ __device__ __forceinline__ void plane_tests(const float4 r, const float (&cx)[K]
   }
 }
 
+// Limits of the waits for copies into shared memory; the second one is the test
+// hook's (the copies withheld).
+constexpr unsigned long long kCopyWaitCycles = 2000000000ull;  // about a second
+constexpr unsigned long long kCopyTestWaitCycles = 20000000ull;
+
+__device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, unsigned long long limit) {
+  const unsigned long long t0 = clock64();
+  for (;;) {
+    uint32_t done;
+    asm volatile(
+        "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
+        : "=r"(done)
+        : "r"(bar)
+        : "memory");
+    if (done) return true;
+    if ((unsigned long long)(clock64() - t0) > limit) return false;
+  }
+}
+
+// hold_copy (test hook): the copies are not issued, so the wait runs out and the
+// timeout path is taken.
 template <bool BF16, bool UNIT, bool COPY, int K>
-__global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StageParams p, PairList L, int total_vpls) {
+__global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StageParams p, PairList L, int total_vpls,
+                                                                       int hold_copy) {
   pdl_wait_and_release();
   note_dispatch_size(p);
   extern __shared__ float4 s_rec[];
@@ -261,7 +283,7 @@ __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StagePara
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(total_vpls * 16)
                    : "memory");
       int base = 0;
-      for (int l = 0; l < p.ll.n_lights; ++l) {
+      for (int l = 0; l < p.ll.n_lights && !hold_copy; ++l) {
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                          (uint32_t)__cvta_generic_to_shared(s_rec + base)),
                      "l"(p.ll.lights[l].records), "r"(p.ll.lights[l].n_vpls * 16), "r"(bar)
@@ -270,35 +292,19 @@ __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StagePara
       }
     }
     __syncthreads();  // the barrier is initialised before anyone waits on it
-    bool ok = false;
-    const unsigned long long t0 = clock64();
-    for (;;) {
-      uint32_t done;
-      asm volatile(
-          "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
-          : "=r"(done)
-          : "r"(bar)
-          : "memory");
-      if (done) {
-        ok = true;
-        break;
-      }
-      if ((unsigned long long)(clock64() - t0) > 2000000000ull) break;  // about a second
-    }
+    const unsigned long long limit = hold_copy ? kCopyTestWaitCycles : kCopyWaitCycles;
+    const bool ok = bar_wait_bounded(bar, limit);
     if (__syncthreads_or(!ok)) {
       if (threadIdx.x == 0 && p.err) raise_error(p.err, DRV_DEVERR_TIMEOUT);
+      // This CTA's caches list nothing: the later passes read every cache's
+      // run, and what stands there is an earlier stage's.
+      const uint32_t n = cache_count(p);
+      for (uint32_t c0 = blockIdx.x * K; c0 < n; c0 += gridDim.x * K)
+        if (threadIdx.x < K && c0 + threadIdx.x < n)
+          *reinterpret_cast<uint2*>(L.info + 2 * (c0 + threadIdx.x)) = make_uint2(0u, 0u);
       // the copies may still be in flight: wait for them once more (bounded)
       // before this CTA's shared memory is released
-      const unsigned long long t1 = clock64();
-      for (;;) {
-        uint32_t done;
-        asm volatile(
-            "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
-            : "=r"(done)
-            : "r"(bar)
-            : "memory");
-        if (done || (unsigned long long)(clock64() - t1) > 2000000000ull) break;
-      }
+      bar_wait_bounded(bar, limit);
       return;
     }
   } else {
@@ -370,7 +376,7 @@ __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StagePara
         const bool over = (uint64_t)base + total > (uint64_t)L.cap;
         L.info[2 * c] = base;
         L.info[2 * c + 1] = over ? kPairOverflow : total;
-          s_base[k] = base;
+        s_base[k] = base;
         s_count[k] = over ? kPairOverflow : total;
       }
     }
@@ -732,20 +738,6 @@ __device__ __forceinline__ void stage_vpls_issue(const StageParams& p, unsigned 
   __syncthreads();  // offsets written, barrier initialised before anyone waits on it
 }
 
-__device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, unsigned long long limit) {
-  const unsigned long long t0 = clock64();
-  for (;;) {
-    uint32_t done;
-    asm volatile(
-        "{\n.reg .pred q;\nmbarrier.try_wait.parity.shared::cta.b64 q, [%1], 0;\nselp.u32 %0, 1, 0, q;\n}\n"
-        : "=r"(done)
-        : "r"(bar)
-        : "memory");
-    if (done) return true;
-    if ((unsigned long long)(clock64() - t0) > limit) return false;
-  }
-}
-
 // Waits (bounded) for the copies; false, for the whole CTA, when the wait ran
 // out: the error is latched and the copies were waited for once more, so that
 // the CTA may release its shared memory.
@@ -789,9 +781,7 @@ __device__ __forceinline__ GatherStart gather_start(const StageParams& p, const 
 // kernel, since the VPLs were written before the light stage began) is
 // shared by all its warps. THREADS only sets the warps per CTA.
 // hold_copy (test hook): the copies are not issued, so the wait runs out
-// after kGatherTestWaitCycles (~10 ms) and the timeout path is taken.
-constexpr unsigned long long kGatherWaitCycles = 2000000000ull;  // about a second
-constexpr unsigned long long kGatherTestWaitCycles = 20000000ull;
+// after kCopyTestWaitCycles (~10 ms) and the timeout path is taken.
 template <int NK, bool BF16, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairList L, uint32_t staged,
                                                             int hold_copy) {
@@ -803,7 +793,7 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
   const int lane = threadIdx.x & 31;
   stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, hold_copy);
   pdl_wait_and_release();
-  if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kGatherTestWaitCycles : kGatherWaitCycles)) return;
+  if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kCopyTestWaitCycles : kCopyWaitCycles)) return;
   const uint32_t n_units = L.counters[kGatherUnitsCounter];
   const uint32_t warps = gridDim.x * (THREADS / 32);
   uint32_t u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
@@ -951,7 +941,7 @@ __global__ void __launch_bounds__(kUnshadowedThreads, 1) unshadowed_kernel(Fused
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the apply's first loads overlap this grid's tail
   note_dispatch_size(p);
   stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, 0);
-  const bool ok = !staged || stage_vpls_wait(p, &s_bar, kGatherWaitCycles);
+  const bool ok = !staged || stage_vpls_wait(p, &s_bar, kCopyWaitCycles);
   const uint32_t n_units = ok ? cache_count(p) * (uint32_t)fp.n_chunks : 0u;
   for (uint32_t u = next_unit(fp.work, lane); u < n_units; u = next_unit(fp.work, lane)) {
     const uint32_t cache = u / (uint32_t)fp.n_chunks;
@@ -1089,7 +1079,7 @@ cudaError_t launch_persistent_after(void (*kernel)(KArgs...), int threads, size_
 // The record cull's instance for one-VPL blocks (unit), records copied from
 // the extraction (copy) and K caches per pass (2, 4 or 8).
 template <bool BF16>
-void (*cull_kernel_for(bool unit, bool copy, int K))(StageParams, PairList, int) {
+void (*cull_kernel_for(bool unit, bool copy, int K))(StageParams, PairList, int, int) {
 #define DRV_CULL_K(U, CP)                                                   \
   (K == 2 ? cull_records_kernel<BF16, U, CP, 2>                             \
           : (K == 8 ? cull_records_kernel<BF16, U, CP, 8> : cull_records_kernel<BF16, U, CP, 4>))
@@ -1170,7 +1160,7 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
     }
     auto kernel = cull_kernel_for<BF16>(unit, copy, K);
     if ((e = set_max_smem(reinterpret_cast<const void*>(kernel), kCullRecMaxSmem)) != cudaSuccess) return e;
-    e = launch_persistent(kernel, kCullRecThreads, rec_smem, s, num_sms, p, L, total_vpls);
+    e = launch_persistent(kernel, kCullRecThreads, rec_smem, s, num_sms, p, L, total_vpls, knobs.cull_wait_test);
   } else {
     const size_t cull_smem = (size_t)words * 2 * sizeof(uint32_t);
     e = launch_persistent(cull_kernel<BF16>, kCullThreads, cull_smem, s, num_sms, p, L);
