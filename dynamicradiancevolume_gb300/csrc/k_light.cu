@@ -793,10 +793,15 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
   const int lane = threadIdx.x & 31;
   stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, hold_copy);
   pdl_wait_and_release();
-  if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kCopyTestWaitCycles : kCopyWaitCycles)) return;
   const uint32_t n_units = L.counters[kGatherUnitsCounter];
   const uint32_t warps = gridDim.x * (THREADS / 32);
   uint32_t u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
+  if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kCopyTestWaitCycles : kCopyWaitCycles)) {
+    // A cache that misses one of its units' sums gets none of them.
+    for (; u < n_units; u += warps)
+      if (lane == 0) L.unit_range[L.units[u].x].y = 0u;
+    return;
+  }
   if (u >= n_units) return;
   uint4 unit = L.units[u];
   GatherStart start = gather_start<BF16>(p, L, unit, lane);
@@ -862,14 +867,14 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
 // entry. A kernel of its own (about 3 us), since to count a cache's finished units
 // in the gather takes a fence, an atomic and a wait for every unit: 58 us for the
 // 3.9 M pairs of a 1080p frame and 456 us for 40 M, against 47 and 363. Bound by
-// the latency of its loads. Nothing is added after a gather whose copies timed out.
+// the latency of its loads. A cache whose units a gather CTA left out (its copies
+// timed out) has no range any more: what stands in the slots is another stage's.
 constexpr int kFinishThreads = 128;
 template <int NK, bool BF16>
 __global__ void __launch_bounds__(kFinishThreads) gather_finish_kernel(StageParams p, PairList L) {
   pdl_wait_and_release();
   const int lane = threadIdx.x & 31;
   const uint32_t n = cache_count(p), warps = gridDim.x * (kFinishThreads / 32);
-  if (p.err && (*p.err & DRV_DEVERR_TIMEOUT)) return;
   for (uint32_t c = blockIdx.x * (kFinishThreads / 32) + (threadIdx.x >> 5); c < n; c += warps) {
     const uint2 range = L.unit_range[c];
     if (range.y < 2u || lane >= NK * 3) continue;

@@ -71,3 +71,30 @@ def test_cull_copy_timeout_lists_nothing(bf16, spec, lib, cuda):
     got = _sorted(p)
     assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
     p.close()
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+def test_stage_after_a_gather_timeout_adds_every_unit(bf16, lib, cuda):
+    """The error word keeps a timeout until the next allocation. A stage that
+    runs well after one that timed out (no allocation between them) adds every
+    cache's light, also that of caches of several units: the timed-out stage
+    added nothing, so the SH are those of one clean stage, bit for bit."""
+    w = pipeline.scaled(W_MULTI_UNIT, precision=abi.PRECISION_BF16 if bf16 else abi.PRECISION_FP32)
+    ref_p, ref_pos, ref_sh = _lit(w, 2, light_path=abi.LIGHT_PATH_SPLIT)
+    assert ref_p.light_pairs() > 512 * ref_p.cache_count()  # caches of several units
+    p = pipeline.Pipeline(pipeline.host_frame(w, 2))
+    p.set_tuning(light_path=abi.LIGHT_PATH_SPLIT, gather_wait_test=1)
+    p.raycast_inputs()
+    p.prepare_and_extract()
+    p.voxelize()
+    p.allocate()
+    p.light()
+    _timed_out(p)
+    assert not _sorted(p, len(ref_pos))[1].any()
+    p.set_tuning(gather_wait_test=0)
+    p.light()
+    _timed_out(p)  # still latched
+    pos, sh = _sorted(p, len(ref_pos))
+    assert np.array_equal(pos, ref_pos) and np.array_equal(sh, ref_sh)
+    p.close()
+    ref_p.close()
