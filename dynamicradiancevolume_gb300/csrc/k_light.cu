@@ -763,7 +763,7 @@ __device__ __forceinline__ GatherStart gather_start(const StageParams& p, const 
   const uint32_t i = unit.y + lane;
   const bool listed = unit.z != kPairOverflow && i < unit.z;
   s.block = listed ? __ldg(L.block + i) : 0u;
-  s.shadow = listed ? __ldg(L.shadow + i) : 0.0f;
+  s.shadow = listed ? L.shadow[i] : 0.0f;  // the cone pass's: see launch_after
   return s;
 }
 
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
         const float shadowing = s_next;
         if (i + 32 < hi) {
           b_next = __ldg(L.block + i + 32);
-          s_next = __ldg(L.shadow + i + 32);
+          s_next = L.shadow[i + 32];
         }
         gather_block_staged<NK, BF16, KAHAN>(p, s_vpl, s_vbase, staged, acc, comp, (int)b, cx, cy, cz, shadowing);
       }

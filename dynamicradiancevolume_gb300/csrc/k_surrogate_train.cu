@@ -469,8 +469,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads, 1)
 // 64 slots was 7 us of latency). The last block sums the losses.
 constexpr int kAdamParams = 32, kAdamGroups = 8;
 __global__ void __launch_bounds__(kAdamParams* kAdamGroups)
-    adam_kernel(float* __restrict__ params, float* __restrict__ m, float* __restrict__ v,
-                const float* __restrict__ grad_slots, const float* __restrict__ loss_slots, int n_slots,
+    adam_kernel(float* __restrict__ params, float* __restrict__ m, float* __restrict__ v, const float* grad_slots,
+                const float* loss_slots, int n_slots,
                 float inv_batch, float lr, float beta1, float beta2, float eps, float bc1, float bc2,
                 float weight_decay, float* __restrict__ loss_out) {
   __shared__ float s_sum[kAdamGroups][kAdamParams];

@@ -101,7 +101,9 @@ __device__ __forceinline__ void pdl_wait_and_release() {
 
 // Host: a launch that may start before the previous kernel of the stream
 // has finished (it must call pdl_wait_and_release before reading that
-// kernel's output).
+// kernel's output, and read that output with plain loads: what is read with
+// __ldg or through a const __restrict__ parameter counts as unchanged for the
+// kernel's whole life, so such a load may be moved over the wait).
 template <typename... KArgs, typename... Args>
 cudaError_t launch_after(void (*kernel)(KArgs...), int blocks, int threads, size_t smem, cudaStream_t s,
                          const Args&... args) {
