@@ -1043,10 +1043,10 @@ drv_status drv_get_cone_voxel_reads(DrvContext* ctx, uint32_t reads[3]) {
   if (!ctx || !reads) return DRV_ERR_INVALID_ARG;
   if (!ctx->tuning.count_voxel_reads)
     return fail(ctx, DRV_ERR_INVALID_ARG, "set DrvTuning.count_voxel_reads before the light stage");
-  uint32_t c[8];
+  uint32_t c[drv::kPairCounters];
   DRV_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->s()));
   DRV_TRY_CUDA(ctx, cudaMemcpy(c, ctx->pairs.counters, sizeof(c), cudaMemcpyDeviceToHost));
-  reads[0] = c[1];
+  reads[0] = c[drv::kLevel0ReadsCounter];
   reads[1] = c[2];
   reads[2] = c[7];
   return DRV_OK;
@@ -1054,10 +1054,10 @@ drv_status drv_get_cone_voxel_reads(DrvContext* ctx, uint32_t reads[3]) {
 
 drv_status drv_get_light_pairs(DrvContext* ctx, uint32_t* pairs) {
   if (!ctx || !pairs) return DRV_ERR_INVALID_ARG;
-  uint32_t n = 0;
+  uint64_t n = 0;
   DRV_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->s()));
-  DRV_TRY_CUDA(ctx, cudaMemcpy(&n, ctx->pairs.counters, 4, cudaMemcpyDeviceToHost));
-  *pairs = n;
+  DRV_TRY_CUDA(ctx, cudaMemcpy(&n, ctx->pairs.counters, 8, cudaMemcpyDeviceToHost));
+  *pairs = (uint32_t)std::min<uint64_t>(n, 0xFFFFFFFFull);
   return DRV_OK;
 }
 

@@ -114,7 +114,8 @@ struct LightScratch {
 // expected step count and width, cls[i]; 0xFF: not traced), so that a
 // warp's lanes march cones of one length that take one sampling path; with
 // the surrogate only the pairs it is not confident about are classified.
-// counters (zeroed before each light stage): [0] pairs claimed, [1] level-0
+// counters (zeroed before each light stage): [0, 1] pairs claimed, 64 bits (a
+// full list's claims are counted on, and may pass 32), [kLevel0ReadsCounter] level-0
 // corner bytes, [2] mip records and [7] plain mip texels the cone pass read
 // (its counting instance only), [3] pairs the surrogate left to the cone
 // ([4] zero), [5] pairs the surrogate evaluated, [6] the cone pass's work cursor,
@@ -130,6 +131,7 @@ constexpr uint32_t kPairOverflow = 0xFFFFFFFFu;
 constexpr int kMaxSplitBlocks = 65536;  // shadow blocks per frame the split stage handles
 constexpr int kConeClasses = 32;
 constexpr int kGatherUnitsCounter = 8 + 2 * kConeClasses;
+constexpr int kLevel0ReadsCounter = kGatherUnitsCounter + 1;
 constexpr int kPairCounters = kGatherUnitsCounter + 8;
 constexpr uint32_t kGatherMinUnit = 64;  // fewest pairs a unit is planned for (a multiple of 32)
 constexpr int kGatherSlotFloats = 27;   // partial sums per unit slot (NK * 3 <= 27)

@@ -119,6 +119,18 @@ __device__ __forceinline__ void gather_block(const StageParams& p, float* acc, f
 constexpr int kCullThreads = 256;
 constexpr int kCullWarps = kCullThreads / 32;
 
+// Claims cache c's run of `total` pairs and writes it: {first, number}, or
+// {first of the slots left, kPairOverflow} when the list has not that many left.
+// 64 bits: the caches beyond a full list are counted too.
+__device__ __forceinline__ uint2 claim_run(const PairList& L, uint32_t c, uint32_t total) {
+  const unsigned long long base =
+      total ? atomicAdd(reinterpret_cast<unsigned long long*>(L.counters), (unsigned long long)total) : 0ull;
+  const uint2 run = make_uint2((uint32_t)min(base, (unsigned long long)L.cap),
+                               base + total > (unsigned long long)L.cap ? kPairOverflow : total);
+  *reinterpret_cast<uint2*>(L.info + 2 * c) = run;
+  return run;
+}
+
 // CTA per cache: contributing blocks -> a contiguous run of the pair list.
 template <bool BF16>
 __global__ void __launch_bounds__(kCullThreads) cull_kernel(StageParams p, PairList L) {
@@ -169,12 +181,9 @@ __global__ void __launch_bounds__(kCullThreads) cull_kernel(StageParams p, PairL
         run += __popc(s_mask[w0 + k]);
       }
     if (threadIdx.x == 0) {
-      const uint32_t base = total ? atomicAdd(L.counters, total) : 0u;
-      const bool over = (uint64_t)base + total > (uint64_t)L.cap;
-      L.info[2 * c] = base;
-      L.info[2 * c + 1] = over ? kPairOverflow : total;
-      s_base = base;
-      s_count = over ? kPairOverflow : total;
+      const uint2 run = claim_run(L, c, total);
+      s_base = run.x;
+      s_count = run.y;
     }
     __syncthreads();
     const uint32_t base = s_base;
@@ -372,12 +381,9 @@ __global__ void __launch_bounds__(kCullRecThreads) cull_records_kernel(StagePara
           run += __popc(s_mask[k * W + w0 + q]);
         }
       if (lane == 0) {
-        const uint32_t base = total ? atomicAdd(L.counters, total) : 0u;
-        const bool over = (uint64_t)base + total > (uint64_t)L.cap;
-        L.info[2 * c] = base;
-        L.info[2 * c + 1] = over ? kPairOverflow : total;
-        s_base[k] = base;
-        s_count[k] = over ? kPairOverflow : total;
+        const uint2 claimed = claim_run(L, c, total);
+        s_base[k] = claimed.x;
+        s_count[k] = claimed.y;
       }
     }
     __syncthreads();
@@ -492,7 +498,7 @@ __global__ void __launch_bounds__(kClassThreads, 8) classify_kernel(StageParams 
   __shared__ uint32_t s_hist[kConeClasses];
   if (threadIdx.x < kConeClasses) s_hist[threadIdx.x] = 0u;
   __syncthreads();
-  const uint32_t n = min(L.counters[0], L.cap);
+  const uint32_t n = pair_count(L);
   // The last blocks list the gather's units beside the others' pairs.
   const uint32_t list_blocks = min((uint32_t)kListBlocks, gridDim.x - 1u), pair_blocks = gridDim.x - list_blocks;
   if (blockIdx.x >= pair_blocks || !list_blocks)
@@ -541,7 +547,7 @@ constexpr int kScatterTile = kScatterPerThread * kClassThreads;
 __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
   pdl_wait_and_release();
   __shared__ uint32_t s_region[kConeClasses], s_hist[kConeClasses], s_pos[kConeClasses];
-  const uint32_t n = min(L.counters[0], L.cap);
+  const uint32_t n = pair_count(L);
   static_assert(kConeClasses == 32, "one warp scans the class totals");
   if (threadIdx.x < 32) {
     // exclusive scan of the class totals: one load per lane, shuffles
@@ -589,7 +595,7 @@ __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
 // Thread per cone over L.order, the listed pairs in cone-class order (with
 // the surrogate, the pairs it left unconfident). COUNT (a separate,
 // measuring instance): the voxel loads of all cones are summed into
-// counters[1] (level-0 corner bytes), [2] (16-byte mip records) and [7]
+// counters[kLevel0ReadsCounter] (level-0 corner bytes), [2] (16-byte mip records) and [7]
 // (plain mip texels).
 // Bound by issue (73% of slots) and the L1's data path (69%: scattered byte and
 // record loads): 1920x1080, 3.9 M cones, 346 -> 286 us with the two-phase march
@@ -635,7 +641,7 @@ __global__ void __launch_bounds__(kConeThreads, 6) cone_kernel(StageParams p, Pa
       c += __shfl_xor_sync(0xffffffffu, c, o);
     }
     if (lane == 0) {
-      atomicAdd(L.counters + 1, a);
+      atomicAdd(L.counters + kLevel0ReadsCounter, a);
       atomicAdd(L.counters + 2, b);
       atomicAdd(L.counters + 7, c);
     }

@@ -219,7 +219,7 @@ struct PairRows {
   PairList L;
   float threshold;
 
-  __device__ uint32_t rows() const { return min(L.counters[0], L.cap); }
+  __device__ uint32_t rows() const { return pair_count(L); }
 
   // Writes the row's 32 inputs; false for an empty list slot (inputs 0).
   __device__ bool features(uint32_t i, const FeatureRow& f) const {

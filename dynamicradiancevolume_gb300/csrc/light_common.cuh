@@ -124,6 +124,11 @@ __device__ __forceinline__ uint32_t cache_count(const StageParams& p) {
   return min((uint32_t)max(p.counter->total_light_cache_count, 0), p.max_caches);
 }
 
+// Pairs in the list (claims beyond its capacity hold none).
+__device__ __forceinline__ uint32_t pair_count(const PairList& L) {
+  return (uint32_t)min(*reinterpret_cast<const unsigned long long*>(L.counters), (unsigned long long)L.cap);
+}
+
 // The stage's first kernel: the dispatch size, where the frame wants it.
 __device__ __forceinline__ void note_dispatch_size(const StageParams& p) {
   if (p.dispatch && blockIdx.x == 0 && threadIdx.x == 0) write_dispatch_size(p.dispatch, p.max_caches);

@@ -601,7 +601,8 @@ drv_status drv_get_tuning(DrvContext* ctx, DrvTuning* tuning);
 
 /* (cache, shadow block) pairs the last split light stage found able to
  * contribute (each traced or evaluated once; those beyond the list's
- * capacity traced by the gather). Synchronises. */
+ * capacity traced by the gather); 0xFFFFFFFF when there are that many or more.
+ * Synchronises. */
 drv_status drv_get_light_pairs(DrvContext* ctx, uint32_t* pairs);
 
 /* Voxel loads of the last split light stage's cone pass run with
