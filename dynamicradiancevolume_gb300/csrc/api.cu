@@ -601,43 +601,47 @@ drv_status reduce_rsms(DrvContext* ctx, int first, int n) {
   }
 }
 
-// The VPLs of lights first .. first + n - 1 (L: the first one's) from their chains.
+// Light li's share of an extraction, from its chain.
+drv_status extract_args(DrvContext* ctx, int li, const DrvSpotLight& L, drv::ExtractArgs& a) {
+  const drv::RsmChain& ch = ctx->rsm[li];
+  if (ch.res0 != L.rsm_render_resolution || ch.n_levels < 1)
+    return fail(ctx, DRV_ERR_INVALID_ARG, "drv_prepare_rsm must run for this light first");
+  const int R = L.rsm_read_resolution;
+  const int read_lod = ilog2(ch.res0 / R);
+  const int shadow_level = read_lod + (int)L.indirect_shadow_lod;
+  if (shadow_level >= ch.n_levels) return fail(ctx, DRV_ERR_INVALID_ARG, "RSM chain too short for the shadow lod");
+  if (L.indirect_shadow_sample_interval < 1) return DRV_ERR_INVALID_ARG;
+  a.L = L;
+  a.R = R;
+  a.flux = ch.flux[read_lod];
+  a.nrm = ch.normal[read_lod];
+  a.dls = ch.dls[read_lod];
+  a.read_half = ch.half(read_lod);
+  a.dls_shadow = ch.dls[shadow_level];
+  a.shadow_half = ch.half(shadow_level);
+  a.vpls = ctx->vpls[li];
+  a.cones = ctx->cones[li];
+  a.records = ctx->vpl_records[li];
+  a.steps = ctx->cone_steps[li];
+  return DRV_OK;
+}
+
+// The VPLs of lights first .. first + n - 1 (lights: the first one's) from their
+// chains; with one that is refused, those of the lights before it.
 drv_status extract_vpls(DrvContext* ctx, int first, int n, const DrvSpotLight* lights) {
   drv::ExtractArgs args[DRV_MAX_LIGHTS] = {};
-  for (int q = 0; q < n; ++q) {
-    const int li = first + q;
-    const DrvSpotLight& L = lights[q];
-    const drv::RsmChain& ch = ctx->rsm[li];
-    if (ch.res0 != L.rsm_render_resolution || ch.n_levels < 1)
-      return fail(ctx, DRV_ERR_INVALID_ARG, "drv_prepare_rsm must run for this light first");
-    const int R = L.rsm_read_resolution;
-    const int read_lod = ilog2(ch.res0 / R);
-    const int shadow_level = read_lod + (int)L.indirect_shadow_lod;
-    if (shadow_level >= ch.n_levels) return fail(ctx, DRV_ERR_INVALID_ARG, "RSM chain too short for the shadow lod");
-    if (L.indirect_shadow_sample_interval < 1) return DRV_ERR_INVALID_ARG;
-    drv::ExtractArgs& a = args[q];
-    a.L = L;
-    a.R = R;
-    a.flux = ch.flux[read_lod];
-    a.nrm = ch.normal[read_lod];
-    a.dls = ch.dls[read_lod];
-    a.read_half = ch.half(read_lod);
-    a.dls_shadow = ch.dls[shadow_level];
-    a.shadow_half = ch.half(shadow_level);
-    a.vpls = ctx->vpls[li];
-    a.cones = ctx->cones[li];
-    a.records = ctx->vpl_records[li];
-    a.steps = ctx->cone_steps[li];
-  }
-  DRV_TRY_CUDA(ctx, drv::launch_extract_vpls(ctx->s(), args, n, ctx->cfg.precision));
-  for (int q = 0; q < n; ++q) {
+  drv_status st = DRV_OK;
+  int count = 0;
+  while (count < n && (st = extract_args(ctx, first + count, lights[count], args[count])) == DRV_OK) ++count;
+  if (count) DRV_TRY_CUDA(ctx, drv::launch_extract_vpls(ctx->s(), args, count, ctx->cfg.precision));
+  for (int q = 0; q < count; ++q) {
     const int li = first + q, R = lights[q].rsm_read_resolution, interval = lights[q].indirect_shadow_sample_interval;
     ctx->n_vpls[li] = R * R;
     ctx->interval[li] = interval;
     ctx->n_cones[li] = (R * R + interval - 1) / interval;
     if (li + 1 > ctx->n_lights) ctx->n_lights = li + 1;
   }
-  return DRV_OK;
+  return st;
 }
 
 }  // namespace
@@ -941,9 +945,16 @@ drv_status drv_frame(DrvContext* ctx, const DrvScene* scene, const DrvGBufferVie
   if (ctx->cfg.indirect_shadow && ctx->tuning.light_path != DRV_LIGHT_PATH_SINGLE)
     st = cuda_check(ctx, cudaMemsetAsync(ctx->pairs.counters, 0, drv::kPairCounters * sizeof(uint32_t), ctx->s()),
                     "clear the pair counters");
-  for (int l = 0; l < n_lights && st == DRV_OK; ++l) st = note_rsm(ctx, l, &lights[l], &rsms[l]);
-  if (st == DRV_OK) st = reduce_rsms(ctx, 0, n_lights);
-  if (st == DRV_OK && n_lights > 0) st = extract_vpls(ctx, 0, n_lights, lights);
+  // With a light that is refused, the lights before it are still prepared and
+  // extracted: a chain that is noted is one that drv_extract_vpls reads.
+  int noted = 0;
+  while (noted < n_lights && st == DRV_OK)
+    if ((st = note_rsm(ctx, noted, &lights[noted], &rsms[noted])) == DRV_OK) ++noted;
+  if (noted) {
+    drv_status got = reduce_rsms(ctx, 0, noted);
+    if (got == DRV_OK) got = extract_vpls(ctx, 0, noted, lights);
+    if (got != DRV_OK) st = got;
+  }
   ctx->cur = ctx->side[1];
   if (st == DRV_OK && ctx->cfg.indirect_shadow) {
     st = drv_voxelize(ctx, scene, vol);
