@@ -58,7 +58,10 @@ StageParams make_stage_params(const DrvConfig& cfg, const DrvVolumeInfo& vol, co
   int base = 0;
   for (int l = 0; l < ll.n_lights; ++l) {
     p.block_base[l] = base;
-    base += p.shadow ? ll.lights[l].n_vpls / ll.lights[l].interval : ll.lights[l].n_vpls;
+    // Without indirect shadow a block is a single VPL, whatever the light's
+    // interval says: every kernel steps through a block by the interval.
+    if (!p.shadow) p.ll.lights[l].interval = 1;
+    base += p.ll.lights[l].n_vpls / p.ll.lights[l].interval;
   }
   for (int l = ll.n_lights; l <= DRV_MAX_LIGHTS; ++l) p.block_base[l] = base;
   p.total_blocks = base;
