@@ -751,12 +751,12 @@ drv_status specular_gather(DrvContext* ctx, const drv::LightLaunch& ll, const Dr
   return st;
 }
 
-// The light stage. In a frame, voxels_ready is an event the voxel build records
-// on another stream (only the kernels that read the voxels wait for it; on
-// success the stream has waited), the pair counters are cleared already
-// (counters_clear) and the stage writes its dispatch size (in_frame).
+// The light stage. In a frame (in_frame) it writes its dispatch size, voxels_ready
+// is an event the voxel build records on another stream (only the kernels that
+// read the voxels wait for it; on success the stream has waited), and the pair
+// counters of a split stage are cleared already (counters_clear).
 drv_status light_caches(DrvContext* ctx, const DrvSpotLight* lights, int32_t n_lights, const DrvVolumeInfo* vol,
-                        const DrvPerFrame* frame, cudaEvent_t voxels_ready, bool in_frame) {
+                        const DrvPerFrame* frame, cudaEvent_t voxels_ready, bool in_frame, bool counters_clear) {
   if (!ctx || !lights || !vol || !frame) return DRV_ERR_INVALID_ARG;
   if (n_lights < 0 || n_lights > ctx->cfg.max_lights) return fail(ctx, DRV_ERR_INVALID_ARG, "bad light count");
   drv::LightLaunch ll{};
@@ -797,7 +797,7 @@ drv_status light_caches(DrvContext* ctx, const DrvSpotLight* lights, int32_t n_l
     knobs.count_voxel_reads = ctx->tuning.count_voxel_reads != 0;
     knobs.cull_wait_test = ctx->tuning.gather_wait_test == 2;
     knobs.gather_wait_test = ctx->tuning.gather_wait_test && !knobs.cull_wait_test;
-    knobs.counters_clear = in_frame;
+    knobs.counters_clear = counters_clear;
     drv::SurrogateArgs sur;
     if (surrogate) {
       sur.weights = ctx->sur_weights;
@@ -863,7 +863,7 @@ drv_status light_caches(DrvContext* ctx, const DrvSpotLight* lights, int32_t n_l
 
 drv_status drv_light_caches(DrvContext* ctx, const DrvSpotLight* lights, int32_t n_lights, const DrvVolumeInfo* vol,
                             const DrvPerFrame* frame) {
-  return light_caches(ctx, lights, n_lights, vol, frame, nullptr, false);
+  return light_caches(ctx, lights, n_lights, vol, frame, nullptr, false, false);
 }
 
 namespace {
@@ -942,14 +942,25 @@ drv_status drv_frame(DrvContext* ctx, const DrvScene* scene, const DrvGBufferVie
   for (int i = 0; i < 2; ++i) DRV_TRY_CUDA(ctx, cudaStreamWaitEvent(ctx->side[i], ctx->fork_ev, 0));
   st = DRV_OK;
   ctx->cur = ctx->side[0];
-  if (ctx->cfg.indirect_shadow && ctx->tuning.light_path != DRV_LIGHT_PATH_SINGLE)
-    st = cuda_check(ctx, cudaMemsetAsync(ctx->pairs.counters, 0, drv::kPairCounters * sizeof(uint32_t), ctx->s()),
-                    "clear the pair counters");
   // With a light that is refused, the lights before it are still prepared and
   // extracted: a chain that is noted is one that drv_extract_vpls reads.
   int noted = 0;
   while (noted < n_lights && st == DRV_OK)
     if ((st = note_rsm(ctx, noted, &lights[noted], &rsms[noted])) == DRV_OK) ++noted;
+  // Only a frame that takes the split stage clears its counters: the others
+  // leave the last split stage's to the calls that report them.
+  bool clear = st == DRV_OK && ctx->tuning.light_path != DRV_LIGHT_PATH_SINGLE;
+  drv::LightLaunch ll{};
+  for (; ll.n_lights < noted && clear; ++ll.n_lights) {
+    const DrvSpotLight& L = lights[ll.n_lights];
+    ll.lights[ll.n_lights].n_vpls = L.rsm_read_resolution * L.rsm_read_resolution;
+    ll.lights[ll.n_lights].interval = L.indirect_shadow_sample_interval;
+    clear = L.indirect_shadow_sample_interval >= 1;
+  }
+  clear = clear && drv::light_split_supported(ctx->cfg, ll);
+  if (clear)
+    st = cuda_check(ctx, cudaMemsetAsync(ctx->pairs.counters, 0, drv::kPairCounters * sizeof(uint32_t), ctx->s()),
+                    "clear the pair counters");
   if (noted) {
     drv_status got = reduce_rsms(ctx, 0, noted);
     if (got == DRV_OK) got = extract_vpls(ctx, 0, noted, lights);
@@ -967,7 +978,7 @@ drv_status drv_frame(DrvContext* ctx, const DrvScene* scene, const DrvGBufferVie
   // both side streams are joined, so that no later call races them.
   for (int i = 0; i < 2; ++i) DRV_TRY_CUDA(ctx, cudaEventRecord(ctx->join_ev[i], ctx->side[i]));
   DRV_TRY_CUDA(ctx, cudaStreamWaitEvent(main, ctx->join_ev[0], 0));
-  if (st == DRV_OK) st = light_caches(ctx, lights, n_lights, vol, f, ctx->join_ev[1], true);
+  if (st == DRV_OK) st = light_caches(ctx, lights, n_lights, vol, f, ctx->join_ev[1], true, clear);
   // On success the light stage has waited for the voxels.
   if (st != DRV_OK) DRV_TRY_CUDA(ctx, cudaStreamWaitEvent(main, ctx->join_ev[1], 0));
   if (st == DRV_OK && ctx->spec_env) st = drv_prepare_specular_envmaps(ctx);  // renderer.cpp:556-558
