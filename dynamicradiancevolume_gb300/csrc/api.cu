@@ -169,6 +169,7 @@ cudaError_t alloc_pairs(Context* c, uint64_t cap) {
   c->pairs.partials = reinterpret_cast<float*>(m + o_partials);
   c->pairs.units = reinterpret_cast<uint4*>(m + o_units);
   c->pairs.cls = reinterpret_cast<uint8_t*>(m + o_cls);
+  c->pairs.unit_slots = (uint32_t)slots;
   c->pairs.cap = (uint32_t)cap;
   return cudaSuccess;
 }

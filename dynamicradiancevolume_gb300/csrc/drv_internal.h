@@ -133,7 +133,8 @@ constexpr int kConeClasses = 32;
 constexpr int kGatherUnitsCounter = 8 + 2 * kConeClasses;
 constexpr int kLevel0ReadsCounter = kGatherUnitsCounter + 1;
 constexpr int kPairCounters = kGatherUnitsCounter + 8;
-constexpr uint32_t kGatherMinUnit = 64;  // fewest pairs a unit is planned for (a multiple of 32)
+constexpr uint32_t kGatherMinUnit = 64;   // fewest pairs of a unit, FP32 entries (a multiple of 32)
+constexpr uint32_t kGatherUnitBF16 = 512;  // pairs of a unit, BF16 entries
 constexpr int kGatherSlotFloats = 27;   // partial sums per unit slot (NK * 3 <= 27)
 struct PairList {
   uint32_t* cache;
@@ -146,11 +147,14 @@ struct PairList {
   uint2* unit_range;     // [max_caches]
   float* partials;       // [gather_unit_slots][kGatherSlotFloats]
   uint4* units;          // [gather_unit_slots]
+  uint32_t unit_slots;
   uint32_t cap;
 };
-// Bound on the gather's units for a pair list of `cap` pairs.
+// Units a pair list of `cap` pairs has room for: units of 512 pairs and each
+// cache's last. The listing takes no smaller units than fit (a slot is 124 bytes:
+// with room for units of 64 pairs, 160 MB for 262144 caches instead of 49).
 inline size_t gather_unit_slots(uint64_t cap, uint32_t max_caches) {
-  return (size_t)(cap / kGatherMinUnit + 1) + max_caches;
+  return (size_t)(cap / kGatherUnitBF16 + 1) + max_caches;
 }
 
 // Ray frame of a pinhole camera: direction = normalize(fwd + nx*right + ny*up).

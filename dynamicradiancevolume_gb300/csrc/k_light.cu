@@ -432,7 +432,6 @@ __device__ __forceinline__ int cone_class(float light_dist, float inv_voxel, con
 
 constexpr int kClassThreads = 256;
 constexpr int kListBlocks = 16;
-constexpr uint32_t kGatherUnitBF16 = 512;
 constexpr int kGatherWarps = 16;  // a gather CTA's (its smaller instance takes the same units)
 
 // Lists the gather units of every cache's run (one unit, without pairs, for a
@@ -446,16 +445,19 @@ constexpr int kGatherWarps = 16;  // a gather CTA's (its smaller instance takes 
 // differs by an FP32 rounding can round to the next BF16 value, so there a
 // cache's sums shall not depend on the other caches (as above: 43 us for 3.9 M
 // pairs against 47, 354 for 40 M against 363). Same pairs, same units: the sums do
-// not depend on scheduling. By every block, or by a thread of the cull, the
+// not depend on scheduling. The units are as many as the list has slots for
+// (total / unit, and one more per cache), which binds long lists of blocks of
+// several VPLs only. By every block, or by a thread of the cull, the
 // listing delays the pairs by 4 us, and 50 with 20 thousand caches.
 template <bool BF16>
 __device__ __forceinline__ void list_gather_units(const StageParams& p, const PairList& L, uint32_t total,
                                                   uint32_t gather_warps, float vpls_per_pair, uint32_t block,
                                                   uint32_t blocks) {
   const float rounds = (float)total / (32.0f * (float)gather_warps);
-  const uint32_t unit =
-      BF16 ? kGatherUnitBF16 : max(kGatherMinUnit, 32u * (uint32_t)ceilf(sqrtf(2.0f * rounds / vpls_per_pair)));
   const uint32_t n_caches = cache_count(p);
+  const uint32_t least = max(kGatherMinUnit, (total / (L.unit_slots - n_caches) + 32u) & ~31u);
+  const uint32_t unit =
+      BF16 ? kGatherUnitBF16 : max(least, 32u * (uint32_t)ceilf(sqrtf(2.0f * rounds / vpls_per_pair)));
   const int lane = threadIdx.x & 31;
   for (uint32_t c0 = block * blockDim.x + (threadIdx.x & ~31u); c0 < n_caches; c0 += blocks * blockDim.x) {
     const uint32_t c = c0 + lane;
