@@ -384,7 +384,7 @@ MeshView mesh_view(const DrvMesh& mesh) {
 // with them).
 cudaError_t raster(cudaStream_t s, const MeshView& m, const float* view_proj, int W, int H, unsigned long long* keys,
                    uint4* big, int num_sms) {
-  const TileQueue queue{keys - 2, big};
+  const TileQueue queue{keys - 2, big, tile_queue_cap(m.nt, num_sms)};
   cudaError_t e = cudaMemsetAsync(queue.head, 0, ((size_t)W * H + 2) * sizeof(unsigned long long), s);
   if (e != cudaSuccess || m.nt <= 0) return e;
   Mat4 M;

@@ -30,7 +30,16 @@ constexpr int kDirectPixels = 512;
 // Triangles a warp sets up at a time (a lane each) before it walks them: 8
 // and 4 measure the same (327 / 332 us), 16 is slower (566 at 256 pixels).
 constexpr int kWarpTris = 8;
-constexpr uint32_t kTileQueueCap = 16384;
+// Entries of the list. A triangle beyond them is walked by the warp that set it up,
+// with seven others'. A mesh of few triangles would leave most warps idle so, and
+// lists them all (up to two entries each, the near plane's cut); from
+// kDirectWarps warps of eight per SM on, only kLongMeshList. Large triangles at
+// 4096^2 with 16384 entries / room for all, ms: 20 thousand 1.10 / 0.64 (of some
+// 600 pixels) and 13.3 / 5.9 (of 16 thousand), 44 thousand 1.40 / 1.35 and 19.6 /
+// 15.9, 56 thousand 1.48 / 1.77 and 21.9 / 21.1, 160 thousand 2.98 / 5.92 and 47 / 81
+// (every tile's warp sets its triangle up again).
+constexpr uint32_t kTileQueueCap = 98304, kLongMeshList = 16384;
+constexpr int kDirectWarps = 36;
 
 // head: entries claimed (upper 24 bits) and tiles claimed (lower 40), zeroed
 // before each pass. Entry: {first tile (low, high word), code, tiles}.
@@ -39,16 +48,20 @@ constexpr uint32_t kTileQueueCap = 16384;
 struct TileQueue {
   unsigned long long* head;
   uint4* entries;
+  uint32_t cap;  // tile_queue_cap
 };
+inline uint32_t tile_queue_cap(int n_triangles, int num_sms) {
+  return n_triangles <= num_sms * kDirectWarps * kWarpTris ? kTileQueueCap : kLongMeshList;
+}
 
 // Lists a triangle; false when the list is full.
 __device__ __forceinline__ bool tile_queue_push(const TileQueue& q, uint32_t code, uint32_t tiles) {
   // Once full, nothing more is added to the head: at most one entry per
   // resident thread beyond the capacity, far from the 24 bits' limit.
-  if ((uint32_t)(__ldcg(q.head) >> 40) >= kTileQueueCap) return false;
+  if ((uint32_t)(__ldcg(q.head) >> 40) >= q.cap) return false;
   const unsigned long long old = atomicAdd(q.head, (1ull << 40) | tiles);
   const uint32_t slot = (uint32_t)(old >> 40);
-  if (slot >= kTileQueueCap) return false;
+  if (slot >= q.cap) return false;
   const unsigned long long first = old & ((1ull << 40) - 1);
   q.entries[slot] = make_uint4((uint32_t)first, (uint32_t)(first >> 32), code, tiles);
   return true;
@@ -63,7 +76,7 @@ __device__ __forceinline__ unsigned long long tile_queue_first(const uint4& e) {
 // search over the entries (listed in the order of their first tiles).
 template <class F>
 __device__ __forceinline__ void tile_queue_share(const TileQueue& q, uint32_t warp, uint32_t n_warps, F&& visit) {
-  const uint32_t n = min((uint32_t)(*q.head >> 40), kTileQueueCap);
+  const uint32_t n = min((uint32_t)(*q.head >> 40), q.cap);
   if (n == 0) return;
   const uint4 last = q.entries[n - 1];
   const unsigned long long total = tile_queue_first(last) + last.w;
