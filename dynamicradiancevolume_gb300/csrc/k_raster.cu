@@ -19,6 +19,7 @@
 // fillrsm.frag at the hit point.
 #include "drv_device.cuh"
 #include "drv_internal.h"
+#include "light_common.cuh"
 #include "tile_queue.cuh"
 
 namespace drv {
@@ -188,14 +189,15 @@ __device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffff
 // go to the tile list for raster_tiles_kernel (figures: tile_queue.cuh). Bound
 // by issue: about 35 instructions per pixel of a bounding box.
 __global__ void __launch_bounds__(256) raster_kernel(MeshView m, Mat4 M, int W, int H,
-                                                     unsigned long long* __restrict__ keys, TileQueue queue) {
+                                                     unsigned long long* __restrict__ keys, TileQueue queue, int per_warp) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int n_warps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpTris; k0 < m.nt; k0 += n_warps * kWarpTris) {
+  for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp; k0 < m.nt; k0 += n_warps * per_warp) {
 #pragma unroll 1
     for (int f = 1; f <= 2; ++f) {  // fan triangle 2: only of a triangle the near plane cuts
       ScreenTri t{};
-      bool walk = lane < kWarpTris && k0 + lane < m.nt && screen_triangle(m, M, k0 + lane, f, W, H, t);
+      bool walk = lane < per_warp && k0 + lane < m.nt && screen_triangle(m, M, k0 + lane, f, W, H, t);
       if (walk && (long long)(t.bx1 - t.bx0 + 1) * (t.by1 - t.by0 + 1) > kDirectPixels)
         walk = !tile_queue_push(queue, 2u * (uint32_t)(k0 + lane) + (uint32_t)(f - 1),
                                 tile_count(t.bx0, t.by0, t.bx1, t.by1));
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(256) raster_kernel(MeshView m, Mat4 M, int W, 
 // The listed triangles, tile by tile.
 __global__ void __launch_bounds__(256) raster_tiles_kernel(MeshView m, Mat4 M, int W, int H,
                                                            unsigned long long* __restrict__ keys, TileQueue queue) {
+  pdl_wait_and_release();
   const int lane = threadIdx.x & 31;
   tile_queue_share(queue, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
                    [&](uint32_t code, uint32_t tile, uint32_t n) {
@@ -291,17 +294,17 @@ __device__ __forceinline__ bool resolve_hit(const MeshView& m, int tri, f3 o, f3
 }
 
 __global__ void __launch_bounds__(256) gbuffer_resolve_kernel(MeshView m, RayFrame rf, Mat4 M, int w, int h,
-                                                              const unsigned long long* __restrict__ keys,
-                                                              DrvGBufferOut out) {
+                                                              const unsigned long long* keys, DrvGBufferOut out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  const float nx = ((x + 0.5f) / w) * 2.0f - 1.0f, ny = ((y + 0.5f) / h) * 2.0f - 1.0f;
+  const f3 d = normalize3(ldf3(rf.fwd) + ldf3(rf.right) * nx + ldf3(rf.up) * ny);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (x >= w || y >= h) return;
   const size_t i = (size_t)y * w + x;
   const unsigned long long key = keys[i];
   f3 p, n, alb;
   bool hit = false;
   if (key) {
-    const float nx = ((x + 0.5f) / w) * 2.0f - 1.0f, ny = ((y + 0.5f) / h) * 2.0f - 1.0f;
-    const f3 d = normalize3(ldf3(rf.fwd) + ldf3(rf.right) * nx + ldf3(rf.up) * ny);
     hit = resolve_hit(m, (int)(key & 0xFFFFFFFFull) - 1, ldf3(rf.origin), d, p, n, alb);
   }
   if (!hit) {
@@ -339,10 +342,11 @@ __device__ __forceinline__ f3 light_ray_dir(const DrvSpotLight& L, float u, floa
   return normalize3(mkf3(c0 / c3, c1 / c3, c2 / c3) - ldf3(L.position));
 }
 
-__global__ void __launch_bounds__(256) rsm_resolve_kernel(MeshView m, DrvSpotLight L,
-                                                          const unsigned long long* __restrict__ keys, DrvRSMOut out) {
+__global__ void __launch_bounds__(256) rsm_resolve_kernel(MeshView m, DrvSpotLight L, const unsigned long long* keys,
+                                                          DrvRSMOut out) {
   const int R = L.rsm_render_resolution;
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (x >= R || y >= R) return;
   const size_t i = (size_t)y * R + x;
   const unsigned long long key = keys[i];
@@ -389,11 +393,11 @@ cudaError_t raster(cudaStream_t s, const MeshView& m, const float* view_proj, in
   if (e != cudaSuccess || m.nt <= 0) return e;
   Mat4 M;
   for (int i = 0; i < 16; ++i) M.m[i] = view_proj[i];
-  const int warps = (m.nt - 1) / kWarpTris + 1 < num_sms * 64 ? (m.nt - 1) / kWarpTris + 1 : num_sms * 64;
-  raster_kernel<<<(warps + 7) / 8, 256, 0, s>>>(m, M, W, H, keys, queue);
+  const int per_warp = warp_triangles(m.nt, num_sms), groups = (m.nt - 1) / per_warp + 1;
+  const int warps = groups < num_sms * 64 ? groups : num_sms * 64;
+  raster_kernel<<<(warps + 7) / 8, 256, 0, s>>>(m, M, W, H, keys, queue, per_warp);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  raster_tiles_kernel<<<num_sms * 6, 256, 0, s>>>(m, M, W, H, keys, queue);
-  return cudaGetLastError();
+  return launch_after(raster_tiles_kernel, num_sms * 6, 256, 0, s, m, M, W, H, keys, queue);
 }
 
 }  // namespace
@@ -406,8 +410,7 @@ cudaError_t launch_raster_gbuffer(cudaStream_t s, const DrvMesh& mesh, RayFrame 
   Mat4 M;
   for (int i = 0; i < 16; ++i) M.m[i] = view_proj[i];
   dim3 block(16, 16), grid((w + 15) / 16, (h + 15) / 16);
-  gbuffer_resolve_kernel<<<grid, block, 0, s>>>(m, rf, M, w, h, keys, out);
-  return cudaGetLastError();
+  return launch_after(gbuffer_resolve_kernel, grid, block, 0, s, m, rf, M, w, h, keys, out);
 }
 
 cudaError_t launch_raster_rsm(cudaStream_t s, const DrvMesh& mesh, const DrvSpotLight& L, unsigned long long* keys,
@@ -417,8 +420,7 @@ cudaError_t launch_raster_rsm(cudaStream_t s, const DrvMesh& mesh, const DrvSpot
   cudaError_t e = raster(s, m, L.view_projection, R, R, keys, big, num_sms);
   if (e != cudaSuccess) return e;
   dim3 block(16, 16), grid((R + 15) / 16, (R + 15) / 16);
-  rsm_resolve_kernel<<<grid, block, 0, s>>>(m, L, keys, out);
-  return cudaGetLastError();
+  return launch_after(rsm_resolve_kernel, grid, block, 0, s, m, L, keys, out);
 }
 
 }  // namespace drv

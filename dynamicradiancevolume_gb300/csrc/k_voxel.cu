@@ -8,6 +8,7 @@
 // 8^l <= 2^24 for N <= 256), so FP32 holds them exactly.
 #include "drv_device.cuh"
 #include "drv_internal.h"
+#include "light_common.cuh"
 #include "tile_queue.cuh"
 
 namespace drv {
@@ -253,18 +254,21 @@ __device__ __forceinline__ void tri_pixel(const TriWalk& t, int px, int py, int 
 __device__ __forceinline__ float bcast(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 __device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 
-// A lane sets up a triangle (grid-stride, kWarpTris per warp); the warp walks
-// the small ones one after the other, the large ones go to the tile list for
-// triangle_tiles_kernel (figures: tile_queue.cuh).
+// A lane sets up a triangle (grid-stride, up to kWarpTris per warp); the warp walks
+// the small ones one after the other, a lane per pixel of the box in turn, the
+// large ones (a box above `direct`) go to the tile list for triangle_tiles_kernel
+// (figures: tile_queue.cuh).
 __global__ void __launch_bounds__(256) triangles_kernel(const float* __restrict__ pos, int n_vertices,
                                                         const uint32_t* __restrict__ idx, int n_tris, TriVolume tv,
-                                                        int N, uint32_t* __restrict__ bits, TileQueue queue) {
+                                                        int N, uint32_t* __restrict__ bits, TileQueue queue,
+                                                        int per_warp, int direct) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int n_warps = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarpTris; k0 < n_tris; k0 += n_warps * kWarpTris) {
+  for (int k0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp; k0 < n_tris; k0 += n_warps * per_warp) {
     TriWalk t{};
-    bool walk = lane < kWarpTris && k0 + lane < n_tris && tri_walk(pos, n_vertices, idx, k0 + lane, tv, N, t);
-    if (walk && (t.x1 - t.x0 + 1) * (t.y1 - t.y0 + 1) > kDirectPixels)
+    bool walk = lane < per_warp && k0 + lane < n_tris && tri_walk(pos, n_vertices, idx, k0 + lane, tv, N, t);
+    if (walk && (t.x1 - t.x0 + 1) * (t.y1 - t.y0 + 1) > direct)
       walk = !tile_queue_push(queue, (uint32_t)(k0 + lane), tile_count(t.x0, t.y0, t.x1, t.y1));
     for (uint32_t todo = __ballot_sync(0xffffffffu, walk); todo; todo &= todo - 1) {
       const int src = __ffs(todo) - 1;
@@ -278,17 +282,16 @@ __global__ void __launch_bounds__(256) triangles_kernel(const float* __restrict_
       b.zA = bcast(t.zA, src), b.zB = bcast(t.zB, src), b.zC = bcast(t.zC, src);
       b.max_change = bcast(t.max_change, src), b.side = bcast(t.side, src);
       b.x0 = bcast(t.x0, src), b.y0 = bcast(t.y0, src), b.x1 = bcast(t.x1, src), b.y1 = bcast(t.y1, src);
-      const int lw = lanes_per_row(b.x1 - b.x0 + 1), lx = lane & (lw - 1), ly = lane / lw;
-      for (int py = b.y0 + ly; py <= b.y1; py += 32 / lw)
-        for (int px = b.x0 + lx; px <= b.x1; px += lw) tri_pixel(b, px, py, N, bits);
+      const int w = b.x1 - b.x0 + 1, total = w * (b.y1 - b.y0 + 1);
+      for (int q = lane; q < total; q += 32) tri_pixel(b, b.x0 + q % w, b.y0 + q / w, N, bits);
     }
   }
 }
 
 // The listed triangles, tile by tile.
-__global__ void __launch_bounds__(256) triangle_tiles_kernel(const float* __restrict__ pos, int n_vertices,
-                                                             const uint32_t* __restrict__ idx, TriVolume tv, int N,
-                                                             uint32_t* __restrict__ bits, TileQueue queue) {
+__global__ void __launch_bounds__(256) triangle_tiles_kernel(const float* pos, int n_vertices, const uint32_t* idx,
+                                                             TriVolume tv, int N, uint32_t* bits, TileQueue queue) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31;
   tile_queue_share(queue, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
                    [&](uint32_t code, uint32_t tile, uint32_t n) {
@@ -623,12 +626,13 @@ cudaError_t launch_voxelize_triangles(cudaStream_t s, const float* positions, in
   cudaError_t e = cudaMemsetAsync(bits, 0, (words + 4) * sizeof(uint32_t), s);
   if (e != cudaSuccess || n_triangles <= 0) return e;
   TriVolume tv{{vol.volume_world_min[0], vol.volume_world_min[1], vol.volume_world_min[2]}, vol.voxel_size_in_world};
-  const int groups = (n_triangles - 1) / kWarpTris + 1;
+  const int per_warp = warp_triangles(n_triangles, num_sms), groups = (n_triangles - 1) / per_warp + 1;
   const int warps = groups < num_sms * 64 ? groups : num_sms * 64;  // <= 64 warps per SM in flight
-  triangles_kernel<<<(warps + 7) / 8, 256, 0, s>>>(positions, n_vertices, indices, n_triangles, tv, n, bits, queue);
+  triangles_kernel<<<(warps + 7) / 8, 256, 0, s>>>(positions, n_vertices, indices, n_triangles, tv, n, bits, queue, per_warp,
+                                                   n_triangles < num_sms * 16 ? kDirectPixels : kDirectVoxels);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  triangle_tiles_kernel<<<num_sms * 6, 256, 0, s>>>(positions, n_vertices, indices, tv, n, bits, queue);
-  return cudaGetLastError();
+  return launch_after(triangle_tiles_kernel, num_sms * 6, 256, 0, s, positions, n_vertices, indices, tv, n, bits,
+                      queue);
 }
 
 size_t tile_queue_bytes() { return (size_t)kTileQueueCap * sizeof(uint4); }

@@ -105,11 +105,11 @@ __device__ __forceinline__ void pdl_wait_and_release() {
 // __ldg or through a const __restrict__ parameter counts as unchanged for the
 // kernel's whole life, so such a load may be moved over the wait).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_after(void (*kernel)(KArgs...), int blocks, int threads, size_t smem, cudaStream_t s,
+cudaError_t launch_after(void (*kernel)(KArgs...), dim3 blocks, dim3 threads, size_t smem, cudaStream_t s,
                          const Args&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)blocks);
-  cfg.blockDim = dim3((unsigned)threads);
+  cfg.gridDim = blocks;
+  cfg.blockDim = threads;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];

@@ -27,9 +27,21 @@ namespace drv {
 // surface were the last to finish).
 constexpr int kTileW = 32, kTileH = 16;
 constexpr int kDirectPixels = 512;
+// Voxels: from 16 triangles per SM on (there are warps enough), as the walk of a
+// voxel column is shorter than a pixel's and a tile's setup longer. 8 thousand
+// triangles with boxes of some 25 x 25 and 75 x 75 at 256^3: 81 and 374 us, 113 and
+// 328 with 512; one thousand: 39 and 108, 35 and 70 with 512.
+constexpr int kDirectVoxels = 4096;
 // Triangles a warp sets up at a time (a lane each) before it walks them: 8
-// and 4 measure the same (327 / 332 us), 16 is slower (566 at 256 pixels).
+// and 4 measure the same (327 / 332 us), 16 is slower (566 at 256 pixels). Fewer
+// where the mesh would leave warps idle (voxels of 8 thousand triangles with boxes
+// of some 8 x 8: 41 us with eight each, 23 with one; a warp each, set up by every
+// lane and without the tile launch: 20).
 constexpr int kWarpTris = 8;
+inline int warp_triangles(int n_triangles, int num_sms) {
+  const int per = (n_triangles - 1) / (num_sms * 64) + 1;
+  return per < kWarpTris ? per : kWarpTris;
+}
 // Entries of the list. A triangle beyond them is walked by the warp that set it up,
 // with seven others'. A mesh of few triangles would leave most warps idle so, and
 // lists them all (up to two entries each, the near plane's cut); from

@@ -55,3 +55,28 @@ def test_each_form_of_the_list_gives_the_same(lib, cuda):
         for a, b in zip(refs, got):
             assert np.array_equal(a, b)
     p.close()
+
+
+@pytest.mark.parametrize("size,copies", [(0.02, (1, 100, 101, 201, 850)), (0.2, (1, 26, 27, 201))])
+def test_triangles_per_warp_give_the_same(size, copies, lib, cuda):
+    """One triangle per warp, two (from 9729 on, 152 SMs x 64 warps), three and eight,
+    and the voxels' walk where it was set up and by tiles (boxes of up to some 50
+    x 50 voxels, listed above 512 or, from 2432 triangles on, above 4096): the same
+    surfaces, so the same images and voxels."""
+    torch = pytest.importorskip("torch")
+    w = pipeline.scaled(pipeline.WORKLOADS["c1_small"], width=217, height=150, rsm_resolution=64, voxel_res=128)
+    p = pipeline.Pipeline(pipeline.host_frame(w, 5))
+    rng = np.random.default_rng(9)
+    tris = (rng.uniform(0.1, 0.9, (97, 1, 3)) + rng.uniform(-size, size, (97, 3, 3))).astype(np.float32)
+    alb = rng.uniform(0.1, 1.0, (97, 3)).astype(np.float32)
+    refs = None
+    for k in copies:
+        flat = np.tile(tris, (k, 1, 1)).reshape(-1, 3)
+        _raster_inputs(p, lib, Mesh(torch, p.device, flat, None, np.tile(alb, (k, 1))))
+        g, r = _snapshot(p)
+        got = [g["depth"], g["normal16"], g["albedo"], *r[0], _gpu_bits(p, flat)]
+        assert g["depth"].any() and got[-1].any()
+        refs = refs or got
+        for a, b in zip(refs, got):
+            assert np.array_equal(a, b)
+    p.close()
