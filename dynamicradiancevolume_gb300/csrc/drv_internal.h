@@ -120,7 +120,8 @@ struct LightScratch {
 // (its counting instance only), [3] pairs the surrogate left to the cone
 // ([4] zero), [5] pairs the surrogate evaluated, [6] the cone pass's work cursor,
 // [8 + c] pairs of class c, [8 + kConeClasses + c] class c's scatter cursor,
-// [kGatherUnitsCounter] the gather units listed in units.
+// [kGatherUnitsCounter] the gather units listed in units, [kTracedUnitsCounter]
+// those listed from its end: the caches the list could not hold.
 // The gather takes a cache's run in equal units (units[u] = {cache, first pair,
 // end, 1 if it is the cache's only one}, listed by the classification, a cache's
 // units next to each other, unit_range[cache] = {first, number}), a warp per unit;
@@ -132,6 +133,7 @@ constexpr int kMaxSplitBlocks = 65536;  // shadow blocks per frame the split sta
 constexpr int kConeClasses = 32;
 constexpr int kGatherUnitsCounter = 8 + 2 * kConeClasses;
 constexpr int kLevel0ReadsCounter = kGatherUnitsCounter + 1;
+constexpr int kTracedUnitsCounter = kGatherUnitsCounter + 2;
 constexpr int kPairCounters = kGatherUnitsCounter + 8;
 constexpr uint32_t kGatherMinUnit = 64;   // fewest pairs of a unit, FP32 entries (a multiple of 32)
 constexpr uint32_t kGatherUnitBF16 = 512;  // pairs of a unit, BF16 entries

@@ -435,7 +435,7 @@ constexpr int kListBlocks = 16;
 constexpr int kGatherWarps = 16;  // a gather CTA's (its smaller instance takes the same units)
 
 // Lists the gather units of every cache's run (one unit, without pairs, for a
-// cache the list could not hold), by `blocks` blocks. A unit costs
+// cache the list could not hold: from the list's end), by `blocks` blocks. A unit costs
 // the gather about one round of 32 pairs of one VPL beside its pairs (its start,
 // reduction and sums), and a warp's last unit leaves it idle for half of one on
 // average: with T rounds a warp and R rounds a unit the pass takes about
@@ -464,7 +464,7 @@ __device__ __forceinline__ void list_gather_units(const StageParams& p, const Pa
     const uint2 info = c < n_caches ? *reinterpret_cast<const uint2*>(L.info + 2 * c) : make_uint2(0u, 0u);
     const uint32_t base = info.x, count = info.y;
     const bool over = count == kPairOverflow;
-    const uint32_t n = over ? 1u : (count + unit - 1) / unit;
+    const uint32_t n = over ? 0u : (count + unit - 1) / unit;
     // one count per warp: the lanes' units follow each other
     uint32_t incl = n;
 #pragma unroll
@@ -476,9 +476,10 @@ __device__ __forceinline__ void list_gather_units(const StageParams& p, const Pa
     if (lane == 31 && incl) first = atomicAdd(L.counters + kGatherUnitsCounter, incl);
     first = __shfl_sync(0xffffffffu, first, 31) + incl - n;
     if (c >= n_caches) continue;
-    L.unit_range[c] = make_uint2(first, n);
+    L.unit_range[c] = make_uint2(first, over ? 1u : n);
     if (over) {
-      L.units[first] = make_uint4(c, 0u, kPairOverflow, 1u);
+      L.units[L.unit_slots - 1u - atomicAdd(L.counters + kTracedUnitsCounter, 1u)] =
+          make_uint4(c, 0u, kPairOverflow, 1u);
       continue;
     }
     const uint32_t pairs = BF16 ? unit : n ? ((count + n - 1) / n + 31u) & ~31u : 0u;
@@ -761,6 +762,20 @@ __device__ __forceinline__ bool stage_vpls_wait(const StageParams& p, uint64_t* 
   return false;
 }
 
+// Units in the order the gather's warps take them: first the caches to be traced,
+// whose units are by far the longest (a millisecond and more), so that no warp
+// takes a second one before every warp has one; among the others, at the places of
+// their caches, some warps took two (half of 33 M pairs beyond the list: 6.3 ms by
+// cull order, 4.8 to 8.8 ms by cache).
+struct GatherOrder {
+  uint32_t traced, count;
+  __device__ __forceinline__ explicit GatherOrder(const PairList& L)
+      : traced(L.counters[kTracedUnitsCounter]), count(traced + L.counters[kGatherUnitsCounter]) {}
+  __device__ __forceinline__ uint32_t slot(const PairList& L, uint32_t u) const {
+    return u < traced ? L.unit_slots - 1u - u : u - traced;
+  }
+};
+
 // Where a unit begins: its cache's position and each lane's first pair.
 struct GatherStart {
   float x, y, z, shadow;
@@ -804,22 +819,23 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
   const int lane = threadIdx.x & 31;
   stage_vpls_issue<BF16>(p, s_vpl, s_vbase, &s_bar, staged, hold_copy);
   pdl_wait_and_release();
-  const uint32_t n_units = L.counters[kGatherUnitsCounter];
+  const GatherOrder order(L);
+  const uint32_t n_units = order.count;
   const uint32_t warps = gridDim.x * (THREADS / 32);
   uint32_t u = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5);
   if (staged && !stage_vpls_wait(p, &s_bar, hold_copy ? kCopyTestWaitCycles : kCopyWaitCycles)) {
     // A cache that misses one of its units' sums gets none of them.
     for (; u < n_units; u += warps)
-      if (lane == 0) L.unit_range[L.units[u].x].y = 0u;
+      if (lane == 0) L.unit_range[L.units[order.slot(L, u)].x].y = 0u;
     return;
   }
   if (u >= n_units) return;
-  uint4 unit = L.units[u];
+  uint4 unit = L.units[order.slot(L, u)];
   GatherStart start = gather_start<BF16>(p, L, unit, lane);
   for (;;) {
     // the next unit's record is loaded while this unit is summed
     const uint32_t u_next = u + warps;
-    const uint4 unit_next = u_next < n_units ? L.units[u_next] : unit;
+    const uint4 unit_next = u_next < n_units ? L.units[order.slot(L, u_next)] : unit;
     const uint32_t hi = unit.z;
     const float cx = start.x, cy = start.y, cz = start.z;
     float acc[NV], comp[NV];
@@ -866,7 +882,7 @@ __global__ void __launch_bounds__(THREADS, 1) gather_kernel(StageParams p, PairL
       if (unit.w)
         add_to_entry<BF16>(p.entries + (size_t)unit.x * p.stride_floats, lane, mine);
       else
-        L.partials[(size_t)u * kGatherSlotFloats + lane] = mine;
+        L.partials[(size_t)(u - order.traced) * kGatherSlotFloats + lane] = mine;
     }
     if (u_next >= n_units) break;
     u = u_next;
