@@ -1233,7 +1233,9 @@ cudaError_t split_variant(cudaStream_t s, const StageParams& p, const PairList& 
                     true, p, L, staged, knobs.gather_wait_test);
   }
   if (e != cudaSuccess) return e;
-  if ((e = launch_grid(gather_finish_kernel<NK, BF16>, kFinishThreads, 0, s, num_sms, 8, true, p, L)) != cudaSuccess)
+  // With no more blocks than a unit takes, every cache has one unit at most.
+  if (p.total_blocks > (int)(BF16 ? kGatherUnitBF16 : kGatherMinUnit) &&
+      (e = launch_grid(gather_finish_kernel<NK, BF16>, kFinishThreads, 0, s, num_sms, 8, true, p, L)) != cudaSuccess)
     return e;
   return end(DRV_LK_GATHER);
 }
