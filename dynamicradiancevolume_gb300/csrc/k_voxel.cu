@@ -622,7 +622,7 @@ cudaError_t launch_voxelize_triangles(cudaStream_t s, const float* positions, in
   // The large triangles' list lies behind the bits: its head is cleared with them.
   const size_t words = (size_t)n * n * (n / 32);
   const TileQueue queue{reinterpret_cast<unsigned long long*>(bits + words), reinterpret_cast<uint4*>(bits + words + 4),
-                        tile_queue_cap(n_triangles, num_sms)};
+                        (uint32_t)n_triangles <= kTileQueueCap ? kTileQueueCap : kLongMeshList};
   cudaError_t e = cudaMemsetAsync(bits, 0, (words + 4) * sizeof(uint32_t), s);
   if (e != cudaSuccess || n_triangles <= 0) return e;
   TriVolume tv{{vol.volume_world_min[0], vol.volume_world_min[1], vol.volume_world_min[2]}, vol.voxel_size_in_world};
