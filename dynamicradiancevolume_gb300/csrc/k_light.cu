@@ -1034,7 +1034,8 @@ __global__ void __launch_bounds__(kThreads, 8) light_kernel(FusedParams fp) {
       if (KAHAN) comp[k * kThreads] = 0.0f;
     }
     auto trace_block = [&](int qb) {
-      const float s = block_cone(p, qb, cx, cy, cz);
+      NoReads reads;
+      const float s = block_cone(p, ViewTableFor<BF16 ? March::kNoUnitPhase : March::kOneLoop>{}, qb, cx, cy, cz, reads);
       const int l = block_light(p, qb);
       const LightArgs& la = p.ll.lights[l];
       const int lb = qb - p.block_base[l];
