@@ -321,8 +321,9 @@ drv_status drv_create(const DrvConfig* cfg, DrvContext** out) {
   }
   if ((e = cudaMalloc(&c->sur_weights, drv::surrogate_weights_bytes())) != cudaSuccess) return bail(e);
   // Pair list of the split light stage: room for 256 contributing shadow
-  // blocks per cache on average (clamped to [2^22, 2^26] pairs, 21 B each:
-  // 88 MB .. 1.4 GB; DrvTuning.pair_capacity grows it); caches beyond a full
+  // blocks per cache on average (clamped to [2^22, 2^26] pairs, 17 B each and
+  // 124 B for every 512 of them and every cache: 72 MB + 124 B per cache .. 1.19
+  // GB at 262144 caches; DrvTuning.pair_capacity grows it); caches beyond a full
   // list are traced by the gather itself, with exact cones also when the
   // surrogate is on.
   if ((e = alloc_pairs(c, std::min<uint64_t>(std::max<uint64_t>((uint64_t)cfg->max_caches * 256u, 1ull << 22),

@@ -94,19 +94,6 @@ __device__ __forceinline__ int select_cascade(const DrvVolumeInfo& v, int n_casc
   return c;
 }
 
-// ComputeAddressVolumeCascadeTransition, lightcache.glsl:125-134.
-__device__ __forceinline__ float cascade_transition(const DrvVolumeInfo& v, int c, const float p[3]) {
-  const DrvCascade& k = v.cascades[c];
-  float a0 = __fsub_rn(k.decision_max[0], p[0]), a1 = __fsub_rn(k.decision_max[1], p[1]),
-        a2 = __fsub_rn(k.decision_max[2], p[2]);
-  float b0 = __fsub_rn(p[0], k.decision_min[0]), b1 = __fsub_rn(p[1], k.decision_min[1]),
-        b2 = __fsub_rn(p[2], k.decision_min[2]);
-  float m = fminf(fminf(fminf(a0, a1), a2), fminf(fminf(b0, b1), b2));
-  float denom = __fmul_rn(k.world_voxel_size, v.cav_transition_zone_size);
-  float t = __fsub_rn(1.0f, __fdiv_rn(m, denom));
-  return fminf(fmaxf(t, 0.0f), 1.0f);
-}
-
 // clamp(ivec3(v), 0, res - 1), ivec3 truncating toward zero (NaN: 0).
 __device__ __forceinline__ int trunc_clamp(float v, int res) {
   return __float2int_rz(fminf(fmaxf(v, 0.0f), (float)(res - 1)));
@@ -143,6 +130,7 @@ __device__ __forceinline__ float div_exact(float x, float d, float inv) {
   return inv != 0.0f ? __fmul_rn(x, inv) : __fdiv_rn(x, d);
 }
 
+// ComputeAddressVolumeCascadeTransition, lightcache.glsl:125-134.
 __device__ __forceinline__ float cascade_transition(const DrvVolumeInfo& v, const CellRecip& r, int c,
                                                    const float p[3]) {
   const DrvCascade& k = v.cascades[c];

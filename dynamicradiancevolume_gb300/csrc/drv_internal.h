@@ -193,7 +193,7 @@ struct Context {
   DrvCacheCounter* counter = nullptr;
   // One allocation: 8 words that no allocation clears ([6] mips ticket, [7]
   // input-check bits), then what each allocation clears in one go: the counter
-  // (4 words), 4 scratch words ([0] alloc ticket, [1] device error bits) and the
+  // (4 words), 4 scratch words ([1] device error bits, the others unused) and the
   // atlas.
   uint32_t* frame_mem = nullptr;
   uint32_t* scratch_words = nullptr;
@@ -356,8 +356,8 @@ struct SurrogateArgs {
 
 // Execution knobs of the split light stage (DrvTuning): CTAs per SM of the
 // cone and gather passes (0: as many as fit), the cull's caches per pass (2,
-// 4 or 8) and the gather's threads per cache (128 or 256), and the cone
-// pass's measuring instance.
+// 4 or 8), the gather's threads per CTA (256 or 512), and the cone pass's
+// measuring instance.
 struct SplitKnobs {
   int cone_ctas_per_sm = 0;
   int gather_ctas_per_sm = 0;

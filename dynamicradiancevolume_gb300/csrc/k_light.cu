@@ -8,7 +8,7 @@
 // consecutive VPLs). A frame has only a few thousand caches, and per cache
 // only a small share of the blocks can contribute at all (a block none of
 // whose VPLs has positive flux and faces the cache adds exactly zero whatever
-// its shadowing), so the stage is split in three steps (five launches):
+// its shadowing), so the stage is split in three steps (six launches):
 //
 //  1. cull_records_kernel (K caches per pass against every VPL's plane
 //     record, staged in shared memory; cull_kernel, a CTA per cache over the
@@ -100,21 +100,6 @@ __device__ __forceinline__ void add_to_entry(float* entry, int k, float v) {
     sh[k] = to_bf16(from_bf16(sh[k]) + v);
   } else {
     entry[sh_offset(k / 3, k % 3)] += v;
-  }
-}
-
-// SH gather of the contributing VPLs of block b with the given shadowing
-// into acc/comp (stride 1: register arrays once inlined).
-template <int NK, bool BF16, bool KAHAN>
-__device__ __forceinline__ void gather_block(const StageParams& p, float* acc, float* comp, int b, float cx, float cy,
-                                             float cz, float shadowing) {
-  const int l = block_light(p, b);
-  const LightArgs& la = p.ll.lights[l];
-  const int lb = b - p.block_base[l];
-  for (int j = 0; j < la.interval; ++j) {
-    const VplData v = load_vpl<BF16>(la.vpls, lb * la.interval + j);
-    const Transfer t = transfer(v, cx, cy, cz);
-    if (contributes(v, t) && flux_ok(p, v)) accumulate<NK, KAHAN>(p.ev, acc, comp, 1, v, t, shadowing);
   }
 }
 

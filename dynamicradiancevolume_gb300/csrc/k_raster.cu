@@ -180,9 +180,6 @@ struct TriEdges {
   }
 };
 
-__device__ __forceinline__ float bcast(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-
 // Visibility pass. A lane sets up a triangle (grid-stride, kWarpTris
 // consecutive triangles per warp: a setup per lane instead of one per warp);
 // the warp then walks the small ones one after the other, and the large ones

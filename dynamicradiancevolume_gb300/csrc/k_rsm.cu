@@ -16,6 +16,21 @@ __device__ __forceinline__ float rsm_at(const void* a, int half, size_t i) {
   return half ? __half2float(static_cast<const __half*>(a)[i]) : static_cast<const float*>(a)[i];
 }
 
+// N lights to a launch of the chain (blockIdx.z) or the extraction (blockIdx.y). A
+// light's own launches fill a fraction of the chip: together, three lights' chains
+// and extractions take the time of one (45 -> 16 us before the production frame's
+// cull). A launch's parameters are copied whole, so one light takes an instance of
+// its own (three small lights called one by one: 15.5 us with room for 16 lights,
+// 12.8 so).
+template <int N>
+struct RsmChainBatch {
+  RsmChainArgs light[N];
+};
+template <int N>
+struct ExtractBatch {
+  ExtractArgs light[N];
+};
+
 // The RSM mip chain, downsamplersm.frag:15-33 per pass res -> res/2: flux =
 // sum of the 2x2 children (textureGather), normal = PackNormal16I(normalize(
 // sum of unpacked normals)), (d, d^2) = mean (linear sample at the shared
@@ -26,22 +41,6 @@ __device__ __forceinline__ float rsm_at(const void* a, int half, size_t i) {
 // form it has in global memory (F32 flux and (d, d^2), packed RG16I
 // normals), so each texel is the one a pass from global memory would give.
 // Every level is written out. P: passes (1..3).
-//
-// N lights to a launch (blockIdx.z; the extraction: blockIdx.y). A light's own
-// launches fill a fraction of the chip: together, three lights' chains and
-// extractions take the time of one (45 -> 16 us before the production frame's
-// cull). A launch's parameters are copied whole, so one light takes an instance of
-// its own (chain and extraction of one small light 4.9 us with room for 16 lights,
-// 4.4 so).
-template <int N>
-struct RsmChainBatch {
-  RsmChainArgs light[N];
-};
-template <int N>
-struct ExtractBatch {
-  ExtractArgs light[N];
-};
-
 template <int P, int N>
 __global__ void __launch_bounds__(256) rsm_chain_kernel(const __grid_constant__ RsmChainBatch<N> batch) {
   const RsmChainArgs& a = batch.light[blockIdx.z];

@@ -185,7 +185,7 @@ __device__ __forceinline__ void st4(float* p, float4 v) { *reinterpret_cast<floa
 
 // One layer forward, 32 samples x 64 units: thread (half, sg, ug) sums the
 // products of samples sg + 8 i and units ug + 16 j over its half of the inputs
-// (16 sums, two 16-byte loads per eight multiply-adds), the halves swap the
+// (16 sums, eight 16-byte loads per 64 multiply-adds), the halves swap the
 // sums of two samples each and finish those: z, then a = GELU(z) and the
 // GELU's derivative.
 template <int K, int LDA>

@@ -251,9 +251,6 @@ __device__ __forceinline__ void tri_pixel(const TriWalk& t, int px, int py, int 
   if ((int)dadd(z, t.max_change) != zi) set_voxel_swizzled(bits, N, t.side, px, py, zi + 1);
 }
 
-__device__ __forceinline__ float bcast(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-__device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
-
 // A lane sets up a triangle (grid-stride, up to kWarpTris per warp); the warp walks
 // the small ones one after the other, a lane per pixel of the box in turn, the
 // large ones (a box above `direct`) go to the tile list for triangle_tiles_kernel

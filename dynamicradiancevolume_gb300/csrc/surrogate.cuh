@@ -44,14 +44,9 @@ constexpr int kOffW4 = kOffB3 + kMlpHidden;
 constexpr int kOffB4 = kOffW4 + kMlpOut * kMlpHidden;
 constexpr int kMlpParams = kOffB4 + kMlpOut;  // 10562
 
-// GELU, sigmoid form, and its derivative (training, FP32).
+// GELU in its sigmoid form: x sigmoid(1.702 x) (training, FP32).
 constexpr float kGeluK = 1.702f;
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + __expf(-x)); }
-__device__ __forceinline__ float gelu(float x) { return x * sigmoidf(kGeluK * x); }
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float s = sigmoidf(kGeluK * x);
-  return s + kGeluK * x * s * (1.0f - s);
-}
 
 // Distance (in voxels) the cone of cacheLightingRSM.comp:195-228 reaches
 // before it stops: min(goal, the distance after max_steps steps). The step

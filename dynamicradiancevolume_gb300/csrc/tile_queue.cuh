@@ -119,6 +119,10 @@ __device__ __forceinline__ uint32_t tile_count(int x0, int y0, int x1, int y1) {
   return (uint32_t)tile_columns(x0, x1) * (uint32_t)((y1 - y0) / kTileH + 1);
 }
 
+// A value of lane src, which set the triangle up.
+__device__ __forceinline__ float bcast(float v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+__device__ __forceinline__ int bcast(int v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
 // Lanes per row when a warp walks a small box of width w: 8, 16 or 32.
 __device__ __forceinline__ int lanes_per_row(int w) { return w <= 8 ? 8 : (w <= 16 ? 16 : 32); }
 

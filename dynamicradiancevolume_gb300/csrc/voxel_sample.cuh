@@ -367,7 +367,9 @@ __device__ __forceinline__ float sample_voxels(const VoxelView& v, float sx, flo
 // distance, front-to-back occlusion, at most max_steps samples. Once the
 // occlusion reaches 1 a further step gives occlusion * (1 - s) + s >= 1 for
 // any sample s in [0, 1], so the clamped result is 0 (to within one rounding)
-// whatever is sampled: the march stops there (the reference marches on).
+// whatever is sampled: the march stops there (the reference marches on). An
+// aperture of one makes the second step infinite: its coordinates saturate and its
+// lod is the last level, so the cone ends with the mean opacity.
 //
 // The radius only grows, so the march is a loop on level 0 and then one on the
 // mips: a warp's lanes stay together within each. On level 0 a step's load is
