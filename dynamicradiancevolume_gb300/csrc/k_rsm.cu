@@ -16,19 +16,15 @@ __device__ __forceinline__ float rsm_at(const void* a, int half, size_t i) {
   return half ? __half2float(static_cast<const __half*>(a)[i]) : static_cast<const float*>(a)[i];
 }
 
-// N lights to a launch of the chain (blockIdx.z) or the extraction (blockIdx.y). A
-// light's own launches fill a fraction of the chip: together, three lights' chains
-// and extractions take the time of one (45 -> 16 us before the production frame's
-// cull). A launch's parameters are copied whole, so one light takes an instance of
-// its own (three small lights called one by one: 15.5 us with room for 16 lights,
-// 12.8 so).
-template <int N>
+// The lights of a launch (blockIdx.z; the extraction: blockIdx.y). A light's own
+// launches fill a fraction of the chip: together, three lights' chains and
+// extractions take the time of one (45 -> 16 us before the production frame's
+// cull).
 struct RsmChainBatch {
-  RsmChainArgs light[N];
+  RsmChainArgs light[DRV_MAX_LIGHTS];
 };
-template <int N>
 struct ExtractBatch {
-  ExtractArgs light[N];
+  ExtractArgs light[DRV_MAX_LIGHTS];
 };
 
 // The RSM mip chain, downsamplersm.frag:15-33 per pass res -> res/2: flux =
@@ -41,8 +37,8 @@ struct ExtractBatch {
 // form it has in global memory (F32 flux and (d, d^2), packed RG16I
 // normals), so each texel is the one a pass from global memory would give.
 // Every level is written out. P: passes (1..3).
-template <int P, int N>
-__global__ void __launch_bounds__(256) rsm_chain_kernel(const __grid_constant__ RsmChainBatch<N> batch) {
+template <int P>
+__global__ void __launch_bounds__(256) rsm_chain_kernel(const __grid_constant__ RsmChainBatch batch) {
   const RsmChainArgs& a = batch.light[blockIdx.z];
   if ((int)blockIdx.x * 32 >= a.res || (int)blockIdx.y * 32 >= a.res) return;  // the grid is the largest light's
   __shared__ float s_flux[2][3][256];
@@ -127,8 +123,8 @@ __device__ __forceinline__ f3 unproject_dir(const DrvSpotLight& L, float u, floa
   return normalize3(mkf3(c0 / c3, c1 / c3, c2 / c3) - ldf3(L.position));
 }
 
-template <bool BF16, int N>
-__global__ void __launch_bounds__(256) extract_kernel(const __grid_constant__ ExtractBatch<N> batch) {
+template <bool BF16>
+__global__ void __launch_bounds__(256) extract_kernel(const __grid_constant__ ExtractBatch batch) {
   const ExtractArgs& a = batch.light[blockIdx.y];
   const DrvSpotLight& L = a.L;
   const int R = a.R, read_half = a.read_half, shadow_half = a.shadow_half;
@@ -222,45 +218,35 @@ __global__ void __launch_bounds__(256) extract_kernel(const __grid_constant__ Ex
   }
 }
 
-template <int N>
-cudaError_t rsm_chain(cudaStream_t s, const RsmChainArgs* lights, int n_lights, int passes) {
-  RsmChainBatch<N> batch{};
+}  // namespace
+
+cudaError_t launch_rsm_chain(cudaStream_t s, const RsmChainArgs* lights, int n_lights, int passes) {
+  if (passes < 1 || passes > 3 || n_lights < 1 || n_lights > DRV_MAX_LIGHTS) return cudaErrorInvalidValue;
+  RsmChainBatch batch{};
   int res = 0;
   for (int l = 0; l < n_lights; ++l) {
     batch.light[l] = lights[l];
     res = lights[l].res > res ? lights[l].res : res;
   }
   const dim3 grid((res + 31) / 32, (res + 31) / 32, n_lights);
-  if (passes == 1) rsm_chain_kernel<1, N><<<grid, 256, 0, s>>>(batch);
-  else if (passes == 2) rsm_chain_kernel<2, N><<<grid, 256, 0, s>>>(batch);
-  else rsm_chain_kernel<3, N><<<grid, 256, 0, s>>>(batch);
+  if (passes == 1) rsm_chain_kernel<1><<<grid, 256, 0, s>>>(batch);
+  else if (passes == 2) rsm_chain_kernel<2><<<grid, 256, 0, s>>>(batch);
+  else rsm_chain_kernel<3><<<grid, 256, 0, s>>>(batch);
   return cudaGetLastError();
 }
 
-template <int N>
-cudaError_t extract(cudaStream_t s, const ExtractArgs* lights, int n_lights, int precision) {
-  ExtractBatch<N> batch{};
+cudaError_t launch_extract_vpls(cudaStream_t s, const ExtractArgs* lights, int n_lights, int precision) {
+  if (n_lights < 1 || n_lights > DRV_MAX_LIGHTS) return cudaErrorInvalidValue;
+  ExtractBatch batch{};
   int n = 0;
   for (int l = 0; l < n_lights; ++l) {
     batch.light[l] = lights[l];
     n = lights[l].R * lights[l].R > n ? lights[l].R * lights[l].R : n;
   }
   const dim3 grid((n + 255) / 256, n_lights);
-  if (precision == DRV_PRECISION_BF16) extract_kernel<true, N><<<grid, 256, 0, s>>>(batch);
-  else extract_kernel<false, N><<<grid, 256, 0, s>>>(batch);
+  if (precision == DRV_PRECISION_BF16) extract_kernel<true><<<grid, 256, 0, s>>>(batch);
+  else extract_kernel<false><<<grid, 256, 0, s>>>(batch);
   return cudaGetLastError();
-}
-
-}  // namespace
-
-cudaError_t launch_rsm_chain(cudaStream_t s, const RsmChainArgs* lights, int n_lights, int passes) {
-  if (passes < 1 || passes > 3 || n_lights < 1 || n_lights > DRV_MAX_LIGHTS) return cudaErrorInvalidValue;
-  return n_lights == 1 ? rsm_chain<1>(s, lights, 1, passes) : rsm_chain<DRV_MAX_LIGHTS>(s, lights, n_lights, passes);
-}
-
-cudaError_t launch_extract_vpls(cudaStream_t s, const ExtractArgs* lights, int n_lights, int precision) {
-  if (n_lights < 1 || n_lights > DRV_MAX_LIGHTS) return cudaErrorInvalidValue;
-  return n_lights == 1 ? extract<1>(s, lights, 1, precision) : extract<DRV_MAX_LIGHTS>(s, lights, n_lights, precision);
 }
 
 }  // namespace drv
