@@ -755,8 +755,8 @@ def cone_roofline(r, cache_peaks, pk, w_name) -> dict:
                     "peak_source": pk["source"] + " (hbm_gbs)",
                     "note": "the voxel pyramid is L2-resident; one ncu capture of this pass read 16.5 MB "
                             "from DRAM per launch (profiles/)"},
-            "note": "the cone pass is bound by issue and the L1 data path (73% and 69% active at 3.9 M cones; 23 of "
-                    "32 lanes active, long_scoreboard the top stall): its loads are a small share of either cache's "
+            "note": "the cone pass is bound by issue and the L1 data path (77% and 67% active over a 1080p "
+                    "frame's three lights; 21 of 32 lanes active, long_scoreboard the top stall): its loads are a small share of either cache's "
                     "throughput",
             "gather": gather_roofline(r, pk)}
 

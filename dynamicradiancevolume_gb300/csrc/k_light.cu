@@ -588,8 +588,8 @@ __global__ void __launch_bounds__(kClassThreads) scatter_kernel(PairList L) {
 // measuring instance): the voxel loads of all cones are summed into
 // counters[kLevel0ReadsCounter] (level-0 corner bytes), [2] (16-byte mip records) and [7]
 // (plain mip texels).
-// Bound by issue (73% of slots) and the L1's data path (69%: scattered byte and
-// record loads): 1920x1080, 3.9 M cones, 346 -> 286 us with the two-phase march
+// Bound by issue (77% of slots) and the L1's data path (67%: scattered byte and
+// record loads; a 1920x1080 frame of three lights): 1920x1080, 3.9 M cones, 346 -> 286 us with the two-phase march
 // on texture coordinates and the corner table (voxel_sample.cuh; 322 -> 264 M
 // warp instructions). Six CTAs per SM (40 registers) against five: 633 / 642 us
 // for the frame; 128-thread CTAs leave the tables less L1 (651 against 642).
@@ -941,7 +941,8 @@ __device__ __forceinline__ void finish_unit(const FusedParams& fp, uint32_t u, u
 // Without indirect shadow a VPL's pair is a test and, if it faces the cache, 27
 // sums: a warp per (cache, chunk of VPLs) unit, the VPLs staged in shared
 // memory as for the gather, the sums in registers (one 512-thread CTA per SM),
-// whole rounds of 32 VPLs that face away skipped. Bound by issue. 1953
+// whole rounds of 32 VPLs that face away skipped. Bound by the latency of a round's
+// chains (issue 51% with 16 warps per SM). 1953
 // caches x 4096 VPLs: 104 us as light_kernel (sums read and written in shared
 // memory for every pair, VPLs from L1) -> about 32 us (the 1280x720 frame 218
 // -> 146 us).

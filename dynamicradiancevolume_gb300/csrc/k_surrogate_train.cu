@@ -308,10 +308,11 @@ __device__ __forceinline__ void grad_tile(const float* d, const float* a, int ha
 
 // A cluster of two CTAs per 64-sample tile (grid-stride over the tiles, the
 // gradients kept in registers): forward, backward, the CTAs' gradients summed
-// through distributed shared memory into the cluster's slot. Bound by shared
-// memory: per 32 samples about 920 k multiply-adds in 4 x 4 (layers) and
-// 8 x 8 (gradients) register tiles, 13 k cycles of 16-byte loads. A step of 4096
-// samples: 164 -> 28.7 us (a thread per sample, every operand a 4-byte shared
+// through distributed shared memory into the cluster's slot. Per 32 samples about
+// 920 k multiply-adds in 4 x 4 (layers) and 8 x 8 (gradients) register tiles. Bound
+// by latency: eight warps per SM issue in 22% of its cycles, waiting for the first
+// loads, shared memory and the layers' barriers; the shared memory's data path is at
+// 25%. A step of 4096 samples: 164 -> 28.4 us (a thread per sample, every operand a 4-byte shared
 // load; the whole step, with Adam and the loss sum).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTrainThreads, 1)
     train_kernel(const float* __restrict__ params, const float* __restrict__ X, const float* __restrict__ Y, int n,
